@@ -103,6 +103,10 @@ template <class P> struct GridP {
   const R *d1, *d2, *d3, *d1s, *d2s, *d3s;
   const R *r1, *r2, *r3, *r1s, *r2s, *r3s;
   const R *s11, *s22, *s33;
+  // complex128 only: the spacings' reciprocal words of exact_div.h (all null when a spacing
+  // is out of its range) and (1/d*s[n] + 1/d*s[n-1]) / d*[n] for n >= 1
+  const uint64_t *q1, *q2, *q3, *q1s, *q2s, *q3s;
+  const R *g1, *g2, *g3;
 };
 
 // the same grid seen by another precision with the same real type (F64 -> F64Q)
@@ -116,6 +120,8 @@ template <class Q, class P> inline GridP<Q> grid_as(const GridP<P>& g)
   q.d1 = g.d1; q.d2 = g.d2; q.d3 = g.d3; q.d1s = g.d1s; q.d2s = g.d2s; q.d3s = g.d3s;
   q.r1 = g.r1; q.r2 = g.r2; q.r3 = g.r3; q.r1s = g.r1s; q.r2s = g.r2s; q.r3s = g.r3s;
   q.s11 = g.s11; q.s22 = g.s22; q.s33 = g.s33;
+  q.q1 = g.q1; q.q2 = g.q2; q.q3 = g.q3; q.q1s = g.q1s; q.q2s = g.q2s; q.q3s = g.q3s;
+  q.g1 = g.g1; q.g2 = g.g2; q.g3 = g.g3;
   return q;
 }
 

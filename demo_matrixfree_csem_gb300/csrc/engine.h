@@ -67,10 +67,14 @@ template <class P> struct SweepP {
   int aphi_fix;             // 1: node sweeps with the conductivity-weighted diagonal (not the reference's)
 };
 
-// one launch per component sweep (pipelined warps, k_lusgs2.cu)
-template <class P>
-void launch_sweep_pipelined(const SweepP<P>& s, int comp, bool fwd, int nslot, cudaStream_t st, int vw,
+// one launch per complex64 component sweep (pipelined warps, k_lusgs2.cu)
+void launch_sweep_pipelined(const SweepP<F32>& s, int comp, bool fwd, int nslot, cudaStream_t st, int vw,
                             int lines_per_cta = 1);
+// one launch per complex128 component sweep (k_lusgs64.cu); aphi: A-phi's edge sweeps. T is
+// nslot tables of sweep64_table_bytes, filled by launch_sweep64_table before the first sweep
+void launch_sweep64(const SweepP<F64>& s, int comp, bool fwd, bool aphi, int nslot, const void* T, cudaStream_t st);
+void launch_sweep64_table(const SweepP<F64>& s, int nslot, void* T, cudaStream_t st);
+size_t sweep64_table_bytes(int n1, int n2, int nK);
 bool sweep_pipelined_fits(int comp, int n1, int n2, int nK);  // the sweep's rows fit one CTA
 // complex64 line-tiled sweeps (k_lusgs3.cu): 32 lines per CTA, rows in warp blocks of at
 // most rows_per_warp (4, 8, 16), vw march positions per step for Ey/Ez (1, 2, 4)

@@ -5,6 +5,7 @@
 #include <utility>
 #include <vector>
 #include "engine_model.h"
+#include "exact_div.h"
 #include "prof.h"
 #include "../../include/csem_host.h"
 
@@ -63,6 +64,19 @@ Model::Model(const csem_grid* gp, int airbc_, int fvm_)
     }
   upload(d64, h64);
   upload(d32, h32);
+  // reciprocal words of the complex128 kernels' exact divisions, and the geometric part of
+  // the sweeps' diagonal per axis, (1/ds[n] + 1/ds[n-1]) / d[n] as the reference rounds it
+  std::vector<uint64_t> hq((size_t)9 * L, 0);
+  bool q_ok = true;
+  for (int a = 0; a < 6; a++)
+    for (int q = 0; q < len[a]; q++) {
+      hq[(size_t)a * L + q] = src[a][q] > 0 ? xd_recip(src[a][q]) : 0;
+      if (!hq[(size_t)a * L + q]) q_ok = false;
+    }
+  for (int a = 0; a < 3; a++)
+    for (int q = 1; q < len[a]; q++)
+      hq[(size_t)(6 + a) * L + q] = xd_bits((1.0 / src[a + 3][q] + 1.0 / src[a + 3][q - 1]) / src[a][q]);
+  upload(q64, hq);
   const long ls[3] = {(long)n1 * (n2 + 1) * (n3f + 1), (long)(n1 + 1) * n2 * (n3f + 1), (long)(n1 + 1) * (n2 + 1) * n3f};
   const double* sg[3] = {G.sigma11, G.sigma22, G.sigma33};
   std::vector<double> s64h;
@@ -90,8 +104,16 @@ Model::Model(const csem_grid* gp, int airbc_, int fvm_)
     g.r1s = dbase + 9 * L; g.r2s = dbase + 10 * L; g.r3s = dbase + 11 * L;
     g.s11 = sbase; g.s22 = sbase + ls[0]; g.s33 = sbase + ls[0] + ls[1];
   };
+  memset(&g64, 0, sizeof(g64));
+  memset(&g32, 0, sizeof(g32));
   fill(g64, d64.as<double>(), s64.as<double>());
   fill(g32, d32.as<float>(), s32.as<float>());
+  const uint64_t* qb = q64.as<uint64_t>();
+  if (q_ok) {
+    g64.q1 = qb; g64.q2 = qb + L; g64.q3 = qb + 2 * L;
+    g64.q1s = qb + 3 * L; g64.q2s = qb + 4 * L; g64.q3s = qb + 5 * L;
+  }
+  g64.g1 = (const double*)(qb + 6 * L); g64.g2 = (const double*)(qb + 7 * L); g64.g3 = (const double*)(qb + 8 * L);
 
   acq.n1 = n1; acq.n2 = n2; acq.n3f = n3f; acq.nb = nb; acq.airbc = airbc; acq.fvm = fvm;
   acq.lEx = lEx; acq.lEy = lEy; acq.lE = lE;
@@ -180,6 +202,11 @@ template <class P> GridP<P> Model::grid_shifted() const
   GridP<P> g = grid<P>();
   const int ks = g.kstart;
   g.d3 += ks; g.d3s += ks; g.r3 += ks; g.r3s += ks;
+  if (g.q3) {
+    g.q3 += ks;
+    g.q3s += ks;
+  }
+  if (g.g3) g.g3 += ks;
   g.s11 += (long)ks * n1 * (n2 + 1);
   g.s22 += (long)ks * (n1 + 1) * n2;
   g.s33 += (long)ks * (n1 + 1) * (n2 + 1);
@@ -392,6 +419,16 @@ int build_sweep_groups_halves(int nslot, const double* iom_of_slot, int ns, int 
 }
 
 template <class P>
+void Ops<P>::diag_table(const SweepP<P>& s, int nslot)
+{
+  if constexpr (P::exact) {
+    const size_t b = sweep64_table_bytes(m->n1, m->n2, s.nK) * nmax;
+    if (tab.bytes < b) tab.alloc(b);
+    launch_sweep64_table(s, nslot, tab.p, st);
+  }
+}
+
+template <class P>
 void Ops<P>::apply_lusgs(const C* X, C* Y, int nslot, const int* sys_list, const SysScal<P>* sc, bool bounds_zero,
                          const SweepGroups* grp)
 {
@@ -457,6 +494,9 @@ void Ops<P>::apply_lusgs(const C* X, C* Y, int nslot, const int* sys_list, const
       return;
     }
   }
+  if constexpr (P::exact) {
+    if (pipelined_sweeps) diag_table(s, nslot);
+  }
   // both schedules visit the points of a sweep in an order that respects every
   // dependency of the lexicographic sweep, so they may be mixed sweep by sweep
   auto sweep = [&](int comp, bool fwd) {
@@ -482,7 +522,8 @@ void Ops<P>::apply_lusgs(const C* X, C* Y, int nslot, const int* sys_list, const
       }
     }
     if (pipelined_sweeps && sweep_pipelined_fits(comp, n1, n2, s.nK)) {
-      launch_sweep_pipelined<P>(s, comp, fwd, nslot, st, sweep_vw, sweep_lines);
+      if constexpr (P::exact) launch_sweep64(s, comp, fwd, false, nslot, tab.p, st);
+      else launch_sweep_pipelined(s, comp, fwd, nslot, st, sweep_vw, sweep_lines);
       return;
     }
     const int nd = sweep_diagonals(comp, n1, n2, s.nK);
@@ -524,17 +565,28 @@ void Ops<P>::apply_aphi(const C* X, C* Y, int nslot, const int* sys_list, const 
   zero(Y, m->lE, nslot, sys_list);
   launch_aphi_div<P>(s, BV.as<C>(), nslot, st);
   CSEM_CUDA_TRY(cudaMemsetAsync(V.p, 0, sizeof(C) * (size_t)m->lv * nslot, st));
-  for (int comp = 0; comp < 3; comp++) {
-    const int nd = sweep_diagonals(comp, n1, n2, n3);
-    for (int t = 2; t < 2 + nd; t++) launch_sweep<P>(s, comp, true, true, t, nslot, st);
+  if constexpr (P::exact) {
+    if (pipelined_sweeps) diag_table(s, nslot);
   }
+  // an edge sweep in one launch where the complex128 pipeline takes it, else by diagonals
+  auto edges = [&](int comp, bool fwd) {
+    if constexpr (P::exact) {
+      if (pipelined_sweeps && sweep_pipelined_fits(comp, n1, n2, n3)) {
+        launch_sweep64(s, comp, fwd, true, nslot, tab.p, st);
+        return;
+      }
+    }
+    const int nd = sweep_diagonals(comp, n1, n2, n3);
+    if (fwd)
+      for (int t = 2; t < 2 + nd; t++) launch_sweep<P>(s, comp, true, true, t, nslot, st);
+    else
+      for (int t = 1 + nd; t >= 2; t--) launch_sweep<P>(s, comp, false, true, t, nslot, st);
+  };
+  for (int comp = 0; comp < 3; comp++) edges(comp, true);
   const int np = phi_diagonals(n1, n2, n3);
   for (int t = 3; t < 3 + np; t++) launch_aphi_phi<P>(s, V.as<C>(), t, nslot, st);
   for (int t = 2 + np; t >= 3; t--) launch_aphi_phi<P>(s, V.as<C>(), -t, nslot, st);
-  for (int comp = 2; comp >= 0; comp--) {
-    const int nd = sweep_diagonals(comp, n1, n2, n3);
-    for (int t = 1 + nd; t >= 2; t--) launch_sweep<P>(s, comp, false, true, t, nslot, st);
-  }
+  for (int comp = 2; comp >= 0; comp--) edges(comp, false);
   launch_aphi_grad<P>(s, V.as<C>(), nslot, st);
 }
 

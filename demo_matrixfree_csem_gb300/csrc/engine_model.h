@@ -59,7 +59,7 @@ class Model {
   float rho_water;
   int N1 = 0, N2 = 0;  // airwave grid
   // device data
-  DevBuf d64, d32, s64, s32, x64, air_i, air_w64, air_w32, sH64, sH32;
+  DevBuf d64, d32, q64, s64, s32, x64, air_i, air_w64, air_w32, sH64, sH32;
   GridP<F64> g64;  // operator view (kstart shift applied inside kernels)
   GridP<F32> g32;
   AirP<F64> a64;
@@ -118,7 +118,7 @@ class Ops {
   Model* m;
   int nmax;
   cudaStream_t st;
-  DevBuf hz0, K, K2, ghx, ghy, cap, V, BV, scal, sb;
+  DevBuf hz0, K, K2, ghx, ghy, cap, V, BV, scal, sb, tab;
   FftPlans* fft;
   // LU-SGS sweeps: true = one pipelined-warp launch per component sweep (k_lusgs2.cu),
   // false = one launch per wavefront diagonal (k_lusgs.cu); both give identical results
@@ -170,6 +170,7 @@ class Ops {
                    bool bounds_zero = false, const SweepGroups* grp = nullptr);
   void apply_aphi(const C* X, C* Y, int nslot, const int* sys_list, const SysScal<P>* sc);
   void zero(C* Y, long n, int nslot, const int* sys_list);
+  void diag_table(const SweepP<P>& s, int nslot);  // complex128: the pipelined sweeps' diagonal table
   int split_ctas() const;  // the split pipelines' grid cap on two streams: split_cap CTAs per SM (0: none)
   ~Ops();
 };

@@ -1,4 +1,4 @@
-// Helpers shared by the LU-SGS component sweeps (k_lusgs2.cu: lockstep row pipelines,
+// Helpers shared by the LU-SGS component sweeps (k_lusgs64.cu, k_lusgs2.cu: lockstep row pipelines,
 // k_lusgs3.cu: line-tiled complex64 sweeps, k_lusgs4.cu: row pipelines over several
 // systems at one frequency): the view of one system's vector on the sweep grid, 1-D
 // spacings, read-only loads, the hand-over between warps and the complex64 linear-form

@@ -236,8 +236,8 @@ void *csem_ctx_stream(csem_ctx *c);
  * options; complex64 results may differ in the last bits between schedules:
  *   "lusgs_pipelined" 1 (default): one launch per LU-SGS component sweep, rows as a
  *                     lockstep pipeline; 0: one launch per wavefront diagonal;
- *   "lusgs_vw"        points per thread and step of the pipelined (and split) sweeps: 1,
- *                     2, 4, or 0 for the default (2 complex64, 1 complex128).
+ *   "lusgs_vw"        points per thread and step of the complex64 pipelined (and split)
+ *                     sweeps: 1, 2, 4, or 0 for the default (2); complex128 takes 1.
  *   "lusgs_lines"     complex64 with lusgs_split 0 only: lines one CTA of the pipelined
  *                     sweeps carries one after the other (1..64), so the row pipeline fills
  *                     and drains once per CTA instead of once per line; 1 (default): one
