@@ -17,6 +17,14 @@ void launch_fdfd(const GridP<P>& g, const SysScal<P>* scal, const typename P::C*
 void launch_fdfd_dot(const GridP<F32>& g, const SysScal<F32>* scal, const float2* X, float2* Y, const float2* ghx,
                      const float2* ghy, int nsys, const int* sys_list, cudaStream_t st, int by, int ctas_per_sm,
                      int kind, const float2* E, double2* part);
+// the stencil's grid: tiles in i and j, chunks of planes and planes per chunk
+struct FdfdShape {
+  int gx, gy, nkc, kchunk;
+};
+FdfdShape fdfd_shape(int n1, int n2, int n3, int nsys, int by, int ctas_per_sm);
+template <>
+void launch_fdfd<F64>(const GridP<F64>& g, const SysScal<F64>* scal, const double2* X, double2* Y, const double2* ghx,
+                      const double2* ghy, int nsys, const int* sys_list, cudaStream_t st, int by, int ctas_per_sm);
 int fdfd_partials(int n1, int n2, int n3, int nsys, int by, int ctas_per_sm);  // CTAs per system of the stencil
 template <class P>
 void launch_hz0(const GridP<P>& g, const SysScal<P>* scal, const typename P::C* X, typename P::C* out,

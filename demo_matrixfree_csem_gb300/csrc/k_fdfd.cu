@@ -299,10 +299,7 @@ int sm_count()
 // SM the grid aims for when it splits the planes into chunks (other than 1..16: 4), which
 // sets the z-block depth. Neither changes any result: every output takes the same
 // operands in the same operations.
-struct FdfdShape {
-  int gx, gy, nkc, kchunk;
-};
-static FdfdShape fdfd_shape(int n1, int n2, int n3, int nsys, int by, int ctas_per_sm)
+FdfdShape fdfd_shape(int n1, int n2, int n3, int nsys, int by, int ctas_per_sm)
 {
   if (by != 4 && by != 16) by = 8;
   if (ctas_per_sm < 1 || ctas_per_sm > 16) ctas_per_sm = 4;
@@ -372,8 +369,6 @@ void launch_hz0(const GridP<P>& g, const SysScal<P>* scal, const typename P::C* 
   count_launch(), k_hz0<P><<<grd, blk, 0, st>>>(g, scal, X, out, sys_list);
 }
 
-template void launch_fdfd<F64>(const GridP<F64>&, const SysScal<F64>*, const double2*, double2*,
-                               const double2*, const double2*, int, const int*, cudaStream_t, int, int);
 template void launch_fdfd<F32>(const GridP<F32>&, const SysScal<F32>*, const float2*, float2*,
                                const float2*, const float2*, int, const int*, cudaStream_t, int, int);
 template void launch_fdfd<F64Q>(const GridP<F64Q>&, const SysScal<F64Q>*, const double2*, double2*,

@@ -102,3 +102,21 @@ def test_pipelined_sweeps_equal_diagonal_sweeps(gpu, tmp_path, shape, airbc, fvm
                     ctx.set_option("lusgs_pipelined", 1)
                     got = apply(iom, v)
                     assert np.array_equal(got.view(np.float64), want.view(np.float64), equal_nan=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("airbc,fvm", [(0, 0), (0, 1)])
+def test_operator_equals_oracle(gpu, tmp_path, airbc, fvm):
+    """Columns on either side of a 31-wide tile, planes on either side of a chunk."""
+    from cases import oracle_for
+    cfg = synthetic.random_small(6, 29, 14, 40, airbc=airbc, fvm=fvm, nb=2)
+    G = synthetic.build_grid(cfg, str(tmp_path))
+    ctx = cs.Ctx(G, airbc, fvm)
+    O = oracle_for(G, cfg.params)
+    O.set_hy_length(False)  # n2 < n3: keep Hy and Hz apart, as the kernel does
+    rng = np.random.default_rng(4)
+    x = rng.standard_normal(ctx.lE) + 1j * rng.standard_normal(ctx.lE)
+    for v in (x, np.where(rng.random(ctx.lE) < 0.9, 0, x), x * 10.0 ** rng.uniform(-320, 150, ctx.lE)):
+        for iom in (cs.iom_of(0.75), complex(1e-7, 5e-6)):
+            O.set_iom(iom)
+            assert np.array_equal(ctx.fdfd_apply(iom, v), O.fdfd(v))
