@@ -31,7 +31,7 @@ struct csem_ctx {
   int lusgs_vw = 0;
   int lusgs_lines = 1;
   int lusgs_systems = 1;
-  bool lusgs_split = true;
+  int lusgs_split = 2;
   bool lusgs_overlap = true;
   bool fused_dots = false;
   bool quick_residual = true;
@@ -52,7 +52,8 @@ template <class P> static void configure(const csem_ctx* c, Ops<P>& o)
   o.sweep_vw = c->lusgs_vw;
   o.sweep_lines = c->lusgs_lines;
   o.sweep_systems = c->lusgs_systems;
-  o.split_sweeps = c->lusgs_split;
+  o.split_sweeps = c->lusgs_split != 0;
+  o.line_sweeps = c->lusgs_split == 2;
   o.split_overlap = c->lusgs_overlap;
   o.fused_dots = c->fused_dots;
   o.split_cap = c->lusgs_cap;
@@ -196,7 +197,8 @@ int csem_ctx_set_option(csem_ctx* c, const char* name, int value)
     if (value != 1 && value != 2 && value != 4) return csem_set_error(CSEM_EINVAL, "lusgs_systems must be 1, 2 or 4");
     c->lusgs_systems = value;
   } else if (!strcmp(name, "lusgs_split")) {
-    c->lusgs_split = value != 0;
+    if (value < 0 || value > 2) return csem_set_error(CSEM_EINVAL, "lusgs_split must be 0, 1 or 2");
+    c->lusgs_split = value;
   } else if (!strcmp(name, "quick_residual")) {
     c->quick_residual = value != 0;
   } else if (!strcmp(name, "fused_dots")) {
@@ -787,13 +789,16 @@ static int op_dev(csem_ctx* c, int which, int prec, int nsys, const double* iom,
       if (o->group_size() > 1) {  // the systems of one frequency, grouped
         std::vector<int> h;
         grp.ns = o->group_size();
-        grp.n = grp.ns == SPLIT_GROUP && o->split_overlap
+        grp.n = o->halves()
                     ? build_sweep_groups_halves(nsys, iom, grp.ns, 4, h, &grp.nA, &grp.ngA)
                     : build_sweep_groups(nsys, iom, grp.ns, h);
+        const size_t at = h.size();
+        if (grp.nA == 0) append_slot_groups(nsys, grp.ns, grp.n, h);
         ensure(c->groups, sizeof(int) * h.size());
         // from pageable memory: staged before the call returns, so h may go
         CSEM_CUDA_TRY(cudaMemcpyAsync(c->groups.p, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice, c->st));
         grp.dev = c->groups.as<int>();
+        grp.of_slot = grp.nA == 0 ? grp.dev + at : nullptr;
       }
       o->apply_lusgs((const float2*)x, (float2*)y, nsys, nullptr, s, false, &grp);
     } else o->apply_aphi((const float2*)x, (float2*)y, nsys, nullptr, s);

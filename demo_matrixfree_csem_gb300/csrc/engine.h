@@ -110,6 +110,16 @@ void launch_split_prep(const SweepP<F32>& s, int comp, bool fwd, int nslot, floa
                        int ngroups, int ns, cudaStream_t st);
 void launch_split_sweep(const SweepP<F32>& s, int comp, bool fwd, int nslot, const float4* SB, long sbs, int vw,
                         int max_ctas, cudaStream_t st);
+// complex64 sweeps as a pass over the points and a chain with a warp per line (k_lusgs6.cu):
+// the pass stores B per slot and w per group (SB, SW: sbs float2, sweep_split_scratch, per
+// slot and per group), the chain reads them. groups: ngroups x SPLIT_GROUP slots of one
+// frequency each (null: each slot a group of its own), group_of[slot] a slot's group (null:
+// the slot)
+void launch_line_pass(const SweepP<F32>& s, int comp, bool fwd, int nslot, float2* SB, float2* SW, long sbs,
+                      const int* groups, int ngroups, cudaStream_t st);
+void launch_sweep_line(const SweepP<F32>& s, int comp, bool fwd, int nslot, const float2* SB, const float2* SW, long sbs,
+                       const int* group_of, cudaStream_t st);
+bool sweep_line_fits(int n1, int n2, int nK);  // the rows' tables and edge columns fit shared memory
 int sm_count();  // multiprocessors of the current device
 long sweep_split_scratch(int n1, int n2, int nK);  // largest component on the sweep grid
 template <class P>

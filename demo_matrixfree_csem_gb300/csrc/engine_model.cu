@@ -328,6 +328,12 @@ template <class P> Ops<P>::~Ops()
   if (aux) cudaStreamDestroy(aux);
 }
 
+template <class P> bool Ops<P>::line_fits() const
+{
+  return !P::exact && split_sweeps && line_sweeps && pipelined_sweeps && !tiled_sweeps &&
+         sweep_line_fits(m->n1, m->n2, m->airbc ? m->n3f : m->n3);
+}
+
 template <class P> int Ops<P>::split_ctas() const { return split_cap > 0 ? split_cap * sm_count() : 0; }
 
 template <class P>
@@ -403,6 +409,15 @@ int build_sweep_groups(int nslot, const double* iom_of_slot, int ns, std::vector
   return ng;
 }
 
+void append_slot_groups(int nslot, int ns, int ngroups, std::vector<int>& out)
+{
+  std::vector<int> of((size_t)nslot, 0);
+  for (int g = 0; g < ngroups; g++)
+    for (int q = 0; q < ns; q++)
+      if (out[(size_t)g * ns + q] >= 0) of[out[(size_t)g * ns + q]] = g;
+  out.insert(out.end(), of.begin(), of.end());
+}
+
 int build_sweep_groups_halves(int nslot, const double* iom_of_slot, int ns, int min_half, std::vector<int>& out,
                               int* nA, int* ngA)
 {
@@ -452,6 +467,21 @@ void Ops<P>::apply_lusgs(const C* X, C* Y, int nslot, const int* sys_list, const
   }
   if (!bounds_zero) zero(Y, m->lE, nslot, sys_list);
   if constexpr (!P::exact) {
+    // the systems of one frequency grouped, where the slots are not numbered within halves
+    const bool g16 = grp && grp->ns == SPLIT_GROUP && grp->n > 0 && grp->nA == 0;
+    if (line_fits()) {
+      const long sbs = sweep_split_scratch(n1, n2, s.nK);
+      if (sb.bytes < sizeof(float4) * (size_t)sbs * nmax) sb.alloc(sizeof(float4) * (size_t)sbs * nmax);
+      float2 *B = sb.as<float2>(), *W = B + (size_t)nslot * sbs;
+      const int* groups = g16 && grp->of_slot ? grp->dev : nullptr;
+      auto one = [&](int comp, bool fwd) {
+        launch_line_pass(s, comp, fwd, nslot, B, W, sbs, groups, groups ? grp->n : 0, st);
+        launch_sweep_line(s, comp, fwd, nslot, B, W, sbs, groups ? grp->of_slot : nullptr, st);
+      };
+      for (int comp = 0; comp < 3; comp++) one(comp, true);
+      for (int comp = 2; comp >= 0; comp--) one(comp, false);
+      return;
+    }
     // split sweeps on two halves of the slots, one per stream, the second starting once the
     // first half's first pass is queued: a half's passes (HBM-bound) then run while the
     // other half's pipelines (hand-over-bound) do

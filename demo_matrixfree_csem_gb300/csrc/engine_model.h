@@ -83,6 +83,7 @@ struct SweepGroups {
   // [nA, nslot); the first ngA groups hold slots of the first half, the others slots of
   // the second, each numbered from the start of its half
   int nA = 0, ngA = 0;
+  const int* of_slot = nullptr;  // device: each slot's group (nA == 0 only)
 };
 
 // Groups of at most ns slots with equal iom (iom_of_slot[2 slot], [2 slot + 1]), the
@@ -94,6 +95,9 @@ int build_sweep_groups(int nslot, const double* iom_of_slot, int ns, std::vector
 // *nA = *ngA = 0. Returns the number of groups.
 int build_sweep_groups_halves(int nslot, const double* iom_of_slot, int ns, int min_half, std::vector<int>& out,
                               int* nA, int* ngA);
+
+// Appends each slot's group to the groups in out, for SweepGroups::of_slot
+void append_slot_groups(int nslot, int ns, int ngroups, std::vector<int>& out);
 
 // Krylov dot products of A's result y to form with it: kind 1 out1 = <y, e>, kind 2
 // out1 = <e, y> and out2 = <y, y> (<a, b> = sum a conj(b)), per slot; partial holds
@@ -134,6 +138,11 @@ class Ops {
   // complex64: each component sweep as a coalesced pass storing every point's (B, w) and a
   // row pipeline that reads them (k_lusgs5.cu); scratch sb holds the pass's output
   bool split_sweeps = true;
+  // split sweeps with a warp per line in the row pipeline's place (k_lusgs6.cu), on one stream
+  bool line_sweeps = true;
+  bool line_fits() const;  // they are on and take this grid
+  // whether the caller should number the groups within two halves of the slots
+  bool halves() const { return split_sweeps && split_overlap && !line_fits(); }
   // split sweeps on two halves of the slots, one on `aux`, so that one half's passes can
   // run while the other half's pipelines do; split_cap > 0 runs the pipelines as that many
   // CTAs per SM, each taking lines in turn (0: one CTA per line)

@@ -272,6 +272,18 @@ template <int VW, class C, int NW> struct HandOffN {
   }
 };
 
+// The order in which the split sweeps' chain (k_lusgs6.cu) works through a line, and in which
+// the pass before it stores the line's entries: strips of 32 march positions, in a strip the
+// rows in sweep order, Rp of them (a lane is back from a strip, and its last column written,
+// before the next one starts; whole chunks of 8), in a row 32 positions.
+__host__ __device__ inline int line_steps(int R) { return R < 33 ? 40 : (R + 7) / 8 * 8; }
+__host__ __device__ inline int line_strips(int M) { return (M + 31) / 32; }
+// entry of march step p and row step rho of a line; S strips of Rp rows
+__host__ __device__ inline size_t line_entry(int S, int Rp, int line, int p, int rho)
+{
+  return (((size_t)line * S + (p >> 5)) * Rp + rho) * 32 + (p & 31);
+}
+
 struct Lin32 {
   float2 B, w;
   float gp, gn;

@@ -202,13 +202,20 @@ void MixedBatch::set_list(const std::vector<int>& l)
     iom_slot[2 * q + 1] = h_iom_[2 * (size_t)l[q] + 1];
   }
   int nA = 0, ngA = 0;
-  const int ng = ns == SPLIT_GROUP && o32.split_overlap
+  const int ng = o32.halves()
                      ? build_sweep_groups_halves((int)l.size(), iom_slot.data(), ns, 4, grph_, &nA, &ngA)
                      : build_sweep_groups((int)l.size(), iom_slot.data(), ns, grph_);
-  // at most nsys groups of SPLIT_GROUP: allocated once, so the address captured graphs use stays
-  if (!grpbuf.p) grpbuf.alloc(sizeof(int) * SPLIT_GROUP * (size_t)nsys);
+  // the slots' groups at a fixed place after the at most nsys groups of SPLIT_GROUP, allocated
+  // once, so that the addresses that captured graphs use stay
+  const size_t at = grph_.size(), of = SPLIT_GROUP * (size_t)nsys;
+  if (nA == 0) {
+    append_slot_groups((int)l.size(), ns, ng, grph_);
+    grph_.insert(grph_.begin() + at, of - at, -1);
+  }
+  if (!grpbuf.p) grpbuf.alloc(sizeof(int) * (of + nsys));
   CSEM_CUDA_TRY(cudaMemcpyAsync(grpbuf.p, grph_.data(), sizeof(int) * grph_.size(), cudaMemcpyHostToDevice, st));
   grp_.dev = grpbuf.as<int>();
+  grp_.of_slot = nA == 0 ? grp_.dev + of : nullptr;
   grp_.n = ng;
   grp_.ns = ns;
   grp_.nA = nA;
@@ -265,7 +272,7 @@ void MixedBatch::outer_update(const std::vector<int>& g, std::vector<double>& rn
 // Autotuner of the complex64 kernel shapes, on the batch's current vectors: each
 // candidate is applied once untimed and once timed with CUDA events on the solver's
 // stream, and the fastest is kept for the rest of this batch.
-//  - LU-SGS: the split sweeps (a coalesced pass and a light row pipeline) at 1, 2, 4
+//  - LU-SGS: the split sweeps with a warp per line, or with a row pipeline at 1, 2, 4
 //    points per thread and step; the one-pass pipelined sweeps at points per thread
 //    (1, 2, 4) x lines per CTA (1, 2, 4), or with 2 (1 or 2 points) or 4 (1 point)
 //    systems of one frequency per CTA;
@@ -296,16 +303,17 @@ int MixedBatch::autotune_lusgs(const std::vector<int>& running)
   o32.tiled_sweeps = false;
   float best_ms = 1e30f;
   int best_vw = 2, best_lines = 1, best_ns = 1;
-  bool best_split = true;
-  for (int split : {1, 0})
+  int best_split = 2;
+  for (int split : {2, 1, 0})
     for (int ns : {1, 2, 4}) {
       if (split && ns > 1) continue;
       o32.split_sweeps = split != 0;
+      o32.line_sweeps = split == 2;
       o32.sweep_systems = ns;
       set_list(running);  // the groups for this candidate (the split pass's, or ns per CTA)
       for (int vw : {1, 2, 4})
         for (int lines : {1, 2, 4}) {
-          if ((split && lines > 1) || (ns > 1 && lines > 1) || (ns == 2 && vw == 4) || (ns == 4 && vw > 1)) continue;
+          if ((split == 2 && vw != 2) || (split && lines > 1) || (ns > 1 && lines > 1) || (ns == 2 && vw == 4) || (ns == 4 && vw > 1)) continue;
           o32.sweep_vw = vw;
           o32.sweep_lines = lines;
           const float ms = time([&]() { o32.apply_lusgs(V(0), V(3), nact, dlist, sc, false, &grp_); });
@@ -314,11 +322,12 @@ int MixedBatch::autotune_lusgs(const std::vector<int>& running)
             best_vw = vw;
             best_lines = lines;
             best_ns = ns;
-            best_split = split != 0;
+            best_split = split;
           }
         }
     }
-  o32.split_sweeps = best_split;
+  o32.split_sweeps = best_split != 0;
+  o32.line_sweeps = best_split == 2;
   o32.sweep_systems = best_ns;
   set_list(running);
   o32.pipelined_sweeps = saved;
@@ -342,7 +351,7 @@ int MixedBatch::autotune_lusgs(const std::vector<int>& running)
   o32.stencil_ctas = best_ctas;
   tuned_lines = best_lines;
   tuned_systems = best_ns;
-  tuned_split = best_split ? 1 : 0;
+  tuned_split = best_split;
   tuned_by = best_by;
   tuned_ctas = best_ctas;
   cudaEventDestroy(e0);

@@ -57,7 +57,7 @@ class MixedBatch {
   int tuned_vw = 0;  // shapes chosen by autotune_lusgs (0: not tuned): sweep width,
   int tuned_lines = 0, tuned_by = 0, tuned_ctas = 0;  // lines per CTA, stencil rows, stencil CTAs per SM
   int tuned_systems = 0;  // systems of one frequency per CTA
-  int tuned_split = -1;   // 1: split sweeps chosen
+  int tuned_split = -1;   // 2: split sweeps with a warp per line, 1: with a row pipeline, 0: one-pass sweeps
   long inner_launch_iters = 0;  // sum over launched iterations of active systems
  private:
   void inner_iteration(int nact, const int* dlist, int preco, int maxiter);

@@ -2,7 +2,7 @@
 
     python -m demo_matrixfree_csem_gb300.opbench --workload marlim_like_96 --op lusgs \
         --prec 32 --nsys 16 --reps 5 [--schedule pipelined|diagonal] [--vw 0|1|2|4] \
-        [--split 1|0] [--overlap 1|0] [--cap N] [--systems 1|2|4] [--lines N] [--tiled 0|1] \
+        [--split 2|1|0] [--overlap 1|0] [--cap N] [--systems 1|2|4] [--lines N] [--tiled 0|1] \
         [--by 4|8|16] [--ctas N]
 
 The schedule flags set the context options of the same names (lusgs_split, lusgs_overlap,
@@ -46,9 +46,9 @@ def main(argv=None) -> None:
     ap.add_argument("--lines", type=int, default=1, help="lines per CTA of the complex64 pipelined sweeps")
     ap.add_argument("--systems", type=int, default=1,
                     help="systems of one frequency per CTA of the complex64 pipelined sweeps (1, 2, 4)")
-    ap.add_argument("--split", type=int, default=1,
-                    help="complex64 LU-SGS as a coalesced (B, w) pass and a light row pipeline (1, the "
-                         "default) or one pass (0)")
+    ap.add_argument("--split", type=int, default=2,
+                    help="complex64 LU-SGS as a coalesced pass and a chain with a warp per line (2, the "
+                         "default) or a row pipeline (1), or one pass (0)")
     ap.add_argument("--overlap", type=int, default=1, help="split sweeps on two streams (1, the default) or one (0)")
     ap.add_argument("--cap", type=int, default=0, help="CTAs per SM of the split pipelines on two streams (0: none)")
     ap.add_argument("--by", type=int, default=8, help="stencil output rows per CTA")

@@ -242,10 +242,11 @@ void *csem_ctx_stream(csem_ctx *c);
  *                     sweeps carries one after the other (1..64), so the row pipeline fills
  *                     and drains once per CTA instead of once per line; 1 (default): one
  *                     line per CTA;
- *   "lusgs_split"     complex64 only. 1 (default): each LU-SGS component sweep runs as
- *                     a coalesced pass that forms every point's b/aii + w (known - cross)
- *                     and w = iwmu/aii (once per point for all the systems of a frequency)
- *                     and a row pipeline that reads them and runs only the dependent chain;
+ *   "lusgs_split"     complex64 only. 2 (default): each LU-SGS component sweep runs as a
+ *                     coalesced pass that forms every point's b/aii + w (known - cross)
+ *                     and, once for the systems of a frequency, w = iwmu/aii, and a chain
+ *                     with a warp per line; 1: the pass and a row pipeline with a thread
+ *                     per row, in the chain's place also where a grid is too large for it;
  *                     0: the one-pass pipelined sweeps. Same values to rounding;
  *   "quick_residual"  1 (default): the batched mixed-precision solve forms its complex128
  *                     residuals r = b - A x with a complex128 stencil that multiplies by
@@ -259,7 +260,8 @@ void *csem_ctx_stream(csem_ctx *c);
  *                     partial per CTA); 0 (default): separate dot-product passes, which
  *                     measured faster (the compensated sums double the stencil's
  *                     instructions). The two partition the sums differently;
- *   "lusgs_overlap"   with lusgs_split 1: 1 (default) runs batches of 8 or more systems
+ *   "lusgs_overlap"   with lusgs_split 1 (the chain with a warp per line is faster on one
+ *                     stream): 1 (default) runs batches of 8 or more systems
  *                     as two halves on two streams, so that one half's passes overlap the
  *                     other half's pipelines; 0: one stream. Same bits either way;
  *   "lusgs_cap"       on two streams, the split pipelines run this many CTAs per SM,
@@ -289,7 +291,7 @@ void *csem_ctx_stream(csem_ctx *c);
  *                     (default);
  *   "autotune"        1: the batched mixed-precision solve times the complex64 kernel
  *                     shapes on its first running systems and keeps the fastest for that
- *                     batch: split or one-pass LU-SGS sweeps, their points per thread
+ *                     batch: the three kinds of LU-SGS sweeps, their points per thread
  *                     (1, 2, 4), lines per CTA (1, 2, 4) and systems per CTA (1, 2, 4), the
  *                     stencil's rows per CTA (4, 8, 16) and plane-chunk
  *                     depth (CTAs per SM 2, 4, 8); 0 (default): the fixed defaults.
