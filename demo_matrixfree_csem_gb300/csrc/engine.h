@@ -21,7 +21,11 @@ void launch_fdfd_dot(const GridP<F32>& g, const SysScal<F32>* scal, const float2
 struct FdfdShape {
   int gx, gy, nkc, kchunk;
 };
-FdfdShape fdfd_shape(int n1, int n2, int n3, int nsys, int by, int ctas_per_sm);
+FdfdShape fdfd_shape(int n1, int n2, int n3, int nsys, int by, int ctas_per_sm, int tile);  // tile: columns in i
+constexpr int FDFD32_TILE = 30;  // of the complex64 stencil
+template <>
+void launch_fdfd<F32>(const GridP<F32>& g, const SysScal<F32>* scal, const float2* X, float2* Y, const float2* ghx,
+                      const float2* ghy, int nsys, const int* sys_list, cudaStream_t st, int by, int ctas_per_sm);
 template <>
 void launch_fdfd<F64>(const GridP<F64>& g, const SysScal<F64>* scal, const double2* X, double2* Y, const double2* ghx,
                       const double2* ghy, int nsys, const int* sys_list, cudaStream_t st, int by, int ctas_per_sm);

@@ -12,7 +12,6 @@
 // (fdfd.c:151-172); k_hz0 provides that Hz plane.
 #include "csem_cuda.cuh"
 #include "engine.h"
-#include "k_dot_common.cuh"
 
 namespace csem {
 
@@ -52,26 +51,11 @@ __device__ __forceinline__ void h_at(const GridP<P>& g, const typename P::C* __r
 // plane). Its column's spacings stay in registers and its element offsets advance by one
 // plane stride per plane; the plane's spacings are uniform loads. H is evaluated exactly
 // as in h_at, so complex128 results keep their bits.
-// resident CTAs per SM the complex64 stencil's register budget is sized for (a build may
-// set CSEM_FDFD_MINB to try others); 544-thread CTAs (BY = 16) get one, i.e. no cap below
-// the 255 registers a thread may hold, as three of them would leave 32 per thread
-#ifndef CSEM_FDFD_MINB
-#define CSEM_FDFD_MINB 3
-#endif
-//
-// EPI > 0 (complex64) folds the Krylov dot products of the result into the pass: EPI 1
-// sums y conj(e) (BiCGStab's v.r0 after v = A p), EPI 2 sums e conj(y) and y conj(y) (s.t
-// and t.t after t = A s), e read at the outputs' own indices. Each thread accumulates as
-// the dot-product kernels do (compensated float pairs), the CTA sums its threads in a
-// fixed tree and order, and writes part[slot][cta] (EPI 2: and part[nslot + slot][cta]),
-// which launch_dot_finish adds up in a fixed order: deterministic, but a different
-// partition of the sum than launch_dot's.
-template <class P, int BY, int EPI>
-__global__ void __launch_bounds__(32 * (BY + 1), sizeof(typename P::R) == 8 || BY >= 16 ? 1 : CSEM_FDFD_MINB)
+template <class P, int BY>
+__global__ void __launch_bounds__(32 * (BY + 1), 1)
 k_fdfd(GridP<P> g, const SysScal<P>* __restrict__ scal, const typename P::C* __restrict__ X,
        typename P::C* __restrict__ Y, const typename P::C* __restrict__ GHX,
-       const typename P::C* __restrict__ GHY, int kchunk, int nkc, const int* __restrict__ sys_list,
-       const typename P::C* __restrict__ E, double2* __restrict__ part)
+       const typename P::C* __restrict__ GHY, int kchunk, int nkc, const int* __restrict__ sys_list)
 {
   typedef typename P::C C;
   typedef typename P::R R;
@@ -88,18 +72,6 @@ k_fdfd(GridP<P> g, const SysScal<P>* __restrict__ scal, const typename P::C* __r
   C* bx = Y + (size_t)sys * g.lE;
   C* by = bx + g.lEx;
   C* bz = by + g.lEy;
-  const C* epx = EPI ? E + (size_t)sys * g.lE : nullptr;  // the dot products' other vector
-  const C* epy = EPI ? epx + g.lEx : nullptr;
-  const C* epz = EPI ? epy + g.lEy : nullptr;
-  DotAcc<P> dacc1, dacc2;
-  auto dot = [&](C y, const C* e, long o) {
-    if constexpr (EPI == 1) {
-      dacc1.add(y, e[o]);
-    } else if constexpr (EPI == 2) {
-      dacc1.add(e[o], y);
-      dacc2.add(y, y);
-    }
-  };
   const C iwmu = scal[sys].iwmu, iom = scal[sys].iom;
   const C* ghx = GHX ? GHX + (size_t)slot * (n1 + 1) * n2 : nullptr;  // ghosts are per slot
   const C* ghy = GHY ? GHY + (size_t)slot * n1 * (n2 + 1) : nullptr;
@@ -209,7 +181,6 @@ k_fdfd(GridP<P> g, const SysScal<P>* __restrict__ scal, const typename P::C* __r
           if (g.fvm) r = cmul<P>(r, rmul<P>(P::mul(P::mul(d1s, d2), d3), iom));
         }
         bx[oEx] = r;
-        if (EPI) dot(r, epx, oEx);
       }
       if (outY) {  // by
         C r = z;
@@ -221,7 +192,6 @@ k_fdfd(GridP<P> g, const SysScal<P>* __restrict__ scal, const typename P::C* __r
           if (g.fvm) r = cmul<P>(r, rmul<P>(P::mul(P::mul(d1, d2s), d3), iom));
         }
         by[oEy] = r;
-        if (EPI) dot(r, epy, oEy);
       }
       if (outZ && kin) {  // bz
         C r = z;
@@ -232,36 +202,12 @@ k_fdfd(GridP<P> g, const SysScal<P>* __restrict__ scal, const typename P::C* __r
           if (g.fvm) r = cmul<P>(r, rmul<P>(P::mul(P::mul(d1, d2), d3s), iom));
         }
         bz[oEz] = r;
-        if (EPI) dot(r, epz, oEz);
       }
     }
     pHx = hx;
     pHy = hy;
     exk = ex1;
     eyk = ey1;
-  }
-  if constexpr (EPI > 0) {
-    __shared__ double2 red[2][BY + 1];
-    const double2 v1 = warp_sum(dacc1.value());
-    const double2 v2 = EPI == 2 ? warp_sum(dacc2.value()) : make_double2(0, 0);
-    if (lane == 0) {
-      red[0][w] = v1;
-      red[1][w] = v2;
-    }
-    __syncthreads();
-    if (w == 0 && lane == 0) {
-      double2 a1 = make_double2(0, 0), a2 = make_double2(0, 0);
-      for (int q = 0; q <= BY; q++) {
-        a1.x = __dadd_rn(a1.x, red[0][q].x);
-        a1.y = __dadd_rn(a1.y, red[0][q].y);
-        a2.x = __dadd_rn(a2.x, red[1][q].x);
-        a2.y = __dadd_rn(a2.y, red[1][q].y);
-      }
-      const int npart = gridDim.x * gridDim.y * nkc, nslot = gridDim.z / nkc;
-      const int cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * kc);
-      part[(size_t)slot * npart + cta] = a1;
-      if (EPI == 2) part[(size_t)(nslot + slot) * npart + cta] = a2;
-    }
   }
 }
 
@@ -299,12 +245,12 @@ int sm_count()
 // SM the grid aims for when it splits the planes into chunks (other than 1..16: 4), which
 // sets the z-block depth. Neither changes any result: every output takes the same
 // operands in the same operations.
-FdfdShape fdfd_shape(int n1, int n2, int n3, int nsys, int by, int ctas_per_sm)
+FdfdShape fdfd_shape(int n1, int n2, int n3, int nsys, int by, int ctas_per_sm, int tile)
 {
   if (by != 4 && by != 16) by = 8;
   if (ctas_per_sm < 1 || ctas_per_sm > 16) ctas_per_sm = 4;
   FdfdShape f;
-  f.gx = (n1 + 1 + 30) / 31;
+  f.gx = (n1 + 1 + tile - 1) / tile;
   f.gy = (n2 + 1 + by - 1) / by;
   const long base = (long)f.gx * f.gy * nsys;
   // split the planes into chunks until about ctas_per_sm CTAs per SM are in the grid
@@ -317,31 +263,15 @@ FdfdShape fdfd_shape(int n1, int n2, int n3, int nsys, int by, int ctas_per_sm)
   return f;
 }
 
-int fdfd_partials(int n1, int n2, int n3, int nsys, int by, int ctas_per_sm)
-{
-  const FdfdShape f = fdfd_shape(n1, n2, n3, nsys, by, ctas_per_sm);
-  return f.gx * f.gy * f.nkc;
-}
-
-template <class P, int BY, int EPI>
+template <class P, int BY>
 static void launch_fdfd_by(const GridP<P>& g, const SysScal<P>* scal, const typename P::C* X, typename P::C* Y,
                            const typename P::C* ghx, const typename P::C* ghy, int nsys, const int* sys_list,
-                           cudaStream_t st, int ctas_per_sm, const typename P::C* E, double2* part)
+                           cudaStream_t st, int ctas_per_sm)
 {
-  const FdfdShape f = fdfd_shape(g.n1, g.n2, g.n3, nsys, BY, ctas_per_sm);
+  const FdfdShape f = fdfd_shape(g.n1, g.n2, g.n3, nsys, BY, ctas_per_sm, 31);
   dim3 blk(32, BY + 1);
   dim3 grd(f.gx, f.gy, nsys * f.nkc);
-  count_launch(), k_fdfd<P, BY, EPI><<<grd, blk, 0, st>>>(g, scal, X, Y, ghx, ghy, f.kchunk, f.nkc, sys_list, E, part);
-}
-
-template <class P, int EPI>
-static void launch_fdfd_epi(const GridP<P>& g, const SysScal<P>* scal, const typename P::C* X, typename P::C* Y,
-                            const typename P::C* ghx, const typename P::C* ghy, int nsys, const int* sys_list,
-                            cudaStream_t st, int by, int ctas_per_sm, const typename P::C* E, double2* part)
-{
-  if (by == 4) launch_fdfd_by<P, 4, EPI>(g, scal, X, Y, ghx, ghy, nsys, sys_list, st, ctas_per_sm, E, part);
-  else if (by == 16) launch_fdfd_by<P, 16, EPI>(g, scal, X, Y, ghx, ghy, nsys, sys_list, st, ctas_per_sm, E, part);
-  else launch_fdfd_by<P, 8, EPI>(g, scal, X, Y, ghx, ghy, nsys, sys_list, st, ctas_per_sm, E, part);
+  count_launch(), k_fdfd<P, BY><<<grd, blk, 0, st>>>(g, scal, X, Y, ghx, ghy, f.kchunk, f.nkc, sys_list);
 }
 
 template <class P>
@@ -349,15 +279,9 @@ void launch_fdfd(const GridP<P>& g, const SysScal<P>* scal, const typename P::C*
                  const typename P::C* ghx, const typename P::C* ghy, int nsys, const int* sys_list,
                  cudaStream_t st, int by, int ctas_per_sm)
 {
-  launch_fdfd_epi<P, 0>(g, scal, X, Y, ghx, ghy, nsys, sys_list, st, by, ctas_per_sm, nullptr, nullptr);
-}
-
-void launch_fdfd_dot(const GridP<F32>& g, const SysScal<F32>* scal, const float2* X, float2* Y, const float2* ghx,
-                     const float2* ghy, int nsys, const int* sys_list, cudaStream_t st, int by, int ctas_per_sm,
-                     int kind, const float2* E, double2* part)
-{
-  if (kind == 2) launch_fdfd_epi<F32, 2>(g, scal, X, Y, ghx, ghy, nsys, sys_list, st, by, ctas_per_sm, E, part);
-  else launch_fdfd_epi<F32, 1>(g, scal, X, Y, ghx, ghy, nsys, sys_list, st, by, ctas_per_sm, E, part);
+  if (by == 4) launch_fdfd_by<P, 4>(g, scal, X, Y, ghx, ghy, nsys, sys_list, st, ctas_per_sm);
+  else if (by == 16) launch_fdfd_by<P, 16>(g, scal, X, Y, ghx, ghy, nsys, sys_list, st, ctas_per_sm);
+  else launch_fdfd_by<P, 8>(g, scal, X, Y, ghx, ghy, nsys, sys_list, st, ctas_per_sm);
 }
 
 template <class P>
@@ -369,8 +293,6 @@ void launch_hz0(const GridP<P>& g, const SysScal<P>* scal, const typename P::C* 
   count_launch(), k_hz0<P><<<grd, blk, 0, st>>>(g, scal, X, out, sys_list);
 }
 
-template void launch_fdfd<F32>(const GridP<F32>&, const SysScal<F32>*, const float2*, float2*,
-                               const float2*, const float2*, int, const int*, cudaStream_t, int, int);
 template void launch_fdfd<F64Q>(const GridP<F64Q>&, const SysScal<F64Q>*, const double2*, double2*,
                                 const double2*, const double2*, int, const int*, cudaStream_t, int, int);
 template void launch_hz0<F64>(const GridP<F64>&, const SysScal<F64>*, const double2*, double2*, int,

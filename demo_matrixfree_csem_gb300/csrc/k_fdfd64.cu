@@ -211,7 +211,7 @@ void launch_fdfd<F64>(const GridP<F64>& g, const SysScal<F64>* scal, const C* X,
                       int nsys, const int* sys_list, cudaStream_t st, int by, int ctas_per_sm)
 {
   if (by != 4 && by != 16) by = 8;
-  const FdfdShape f = fdfd_shape(g.n1, g.n2, g.n3, nsys, by, ctas_per_sm);
+  const FdfdShape f = fdfd_shape(g.n1, g.n2, g.n3, nsys, by, ctas_per_sm, 31);
   dim3 blk(32, by + 1), grd(f.gx, f.gy, nsys * f.nkc);
   count_launch();
   if (by == 4) k_fdfd64<4><<<grd, blk, 0, st>>>(g, scal, X, Y, ghx, ghy, f.kchunk, f.nkc, sys_list);
