@@ -10,6 +10,7 @@
 //   F32  fast complex64 for the inner solves of the mixed-precision solver: spacings
 //        enter as precomputed reciprocals, FMA contraction is allowed.
 #pragma once
+#include <atomic>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "prof.h"
@@ -135,5 +136,20 @@ template <class P> struct SysScal {
   typename P::C iom;
   typename P::C iwmu;
 };
+
+constexpr size_t SMEM_MOST = 227 * 1024;
+
+// dynamic shared memory above 48 KB has to be asked for, once per kernel and device
+template <auto KERNEL> inline void allow_smem(size_t bytes)
+{
+  static std::atomic<unsigned long long> done{0};
+  if (bytes <= 48 * 1024) return;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+  if (bit && (done.load(std::memory_order_acquire) & bit)) return;
+  if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MOST) == cudaSuccess)
+    done.fetch_or(bit, std::memory_order_release);
+}
 
 }  // namespace csem

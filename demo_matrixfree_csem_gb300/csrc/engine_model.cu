@@ -155,10 +155,16 @@ Model::Model(const csem_grid* gp, int airbc_, int fvm_)
         wh.push_back(w);
       }
     };
+    const size_t back0 = ih.size();
     back(G.x1, n1 + 1, G.d1fft);
     back(G.x2s, n2, G.d2fft);
     back(G.x1s, n1, G.d1fft);
     back(G.x2, n2 + 1, G.d2fft);
+    // the line transforms take a node past the uniform grid as zero, k_air_scatter the next
+    // row's first: the same where its weight is rounding
+    air_lines = airwave32_fits(n1, n2, N1, N2);
+    for (size_t q = back0; q < ih.size(); q++)
+      if (ih[q] < 0 || ih[q] >= N1 || (ih[q] == N1 - 1 && fabs(wh[q]) > 1e-9)) air_lines = false;
     upload(air_i, ih);
     upload(air_w64, wh);
     std::vector<float> wf(wh.begin(), wh.end());
@@ -169,9 +175,11 @@ Model::Model(const csem_grid* gp, int airbc_, int fvm_)
     for (long q = 0; q < NN; q++) {
       f64[q] = make_double2(G.sH1[2 * q], G.sH1[2 * q + 1]);
       f64[NN + q] = make_double2(G.sH2[2 * q], G.sH2[2 * q + 1]);
-      f32[q] = make_float2((float)G.sH1[2 * q], (float)G.sH1[2 * q + 1]);
-      f32[NN + q] = make_float2((float)G.sH2[2 * q], (float)G.sH2[2 * q + 1]);
+      const long t = air_lines ? q % N1 * N2 + q / N1 : q;
+      f32[t] = make_float2((float)f64[q].x, (float)f64[q].y);
+      f32[NN + t] = make_float2((float)f64[NN + q].x, (float)f64[NN + q].y);
     }
+    if (air_lines) upload(air_tw, air_twiddles(N1));
     upload(sH64, f64);
     upload(sH32, f32);
     auto afill = [&](auto& a, auto* w, auto* sh) {
@@ -304,9 +312,14 @@ Ops<P>::Ops(Model* m_, int nslot_max, cudaStream_t st_) : m(m_), nmax(nslot_max)
 {
   const size_t cs = sizeof(C);
   if (m->airbc) {
-    hz0.alloc(cs * (size_t)m->n1 * m->n2 * nmax);
-    K.alloc(cs * (size_t)m->N1 * m->N2 * nmax);
-    K2.alloc(cs * (size_t)m->N1 * m->N2 * nmax * 2);
+    if (!P::exact && m->air_lines) {  // rows of the model, not of the uniform grid
+      K.alloc(cs * (size_t)m->N1 * m->n2 * nmax);
+      K2.alloc(cs * (size_t)m->N1 * (2 * m->n2 + 1) * nmax);
+    } else {
+      hz0.alloc(cs * (size_t)m->n1 * m->n2 * nmax);
+      K.alloc(cs * (size_t)m->N1 * m->N2 * nmax);
+      K2.alloc(cs * (size_t)m->N1 * m->N2 * nmax * 2);
+    }
     ghx.alloc(cs * (size_t)(m->n1 + 1) * m->n2 * nmax);
     ghy.alloc(cs * (size_t)m->n1 * (m->n2 + 1) * nmax);
     const long capE = (long)m->nb * ((long)m->n1 * (m->n2 + 1) + (long)(m->n1 + 1) * m->n2 + (long)(m->n1 + 1) * (m->n2 + 1));
@@ -353,12 +366,21 @@ bool Ops<P>::apply_A(const C* X, C* Y, int nslot, const int* sys_list, const Sys
   if (m->airbc) {
     const AirP<P>& a = m->air<P>();
     ProfScope air(P::exact ? PROF_AIR64 : PROF_AIR32, st, nslot);
-    launch_hz0<P>(g, sc, X, hz0.as<C>(), nslot, sys_list, st);
-    launch_air_gather<P>(a, hz0.as<C>(), K.as<C>(), nslot, st);
-    fft->exec(P::exact, K.p, nslot, CUFFT_FORWARD, st);
-    launch_air_filter<P>(a, K.as<C>(), K2.as<C>(), nslot, st);
-    fft->exec(P::exact, K2.p, 2 * nslot, CUFFT_INVERSE, st);
-    launch_air_scatter<P>(a, K2.as<C>(), ghx.as<C>(), ghy.as<C>(), nslot, st);
+    bool lines = false;
+    if constexpr (!P::exact) {
+      if ((lines = m->air_lines)) {
+        launch_airwave32(g, a, sc, X, sys_list, m->air_tw.template as<C>(), K.as<C>(), K2.as<C>(), ghx.as<C>(),
+                         ghy.as<C>(), nslot, st);
+      }
+    }
+    if (!lines) {
+      launch_hz0<P>(g, sc, X, hz0.as<C>(), nslot, sys_list, st);
+      launch_air_gather<P>(a, hz0.as<C>(), K.as<C>(), nslot, st);
+      fft->exec(P::exact, K.p, nslot, CUFFT_FORWARD, st);
+      launch_air_filter<P>(a, K.as<C>(), K2.as<C>(), nslot, st);
+      fft->exec(P::exact, K2.p, 2 * nslot, CUFFT_INVERSE, st);
+      launch_air_scatter<P>(a, K2.as<C>(), ghx.as<C>(), ghy.as<C>(), nslot, st);
+    }
     ghxp = ghx.as<C>();
     ghyp = ghy.as<C>();
   }

@@ -59,12 +59,15 @@ class Model {
   float rho_water;
   int N1 = 0, N2 = 0;  // airwave grid
   // device data
-  DevBuf d64, d32, q64, s64, s32, x64, air_i, air_w64, air_w32, sH64, sH32;
+  DevBuf d64, d32, q64, s64, s32, x64, air_i, air_w64, air_w32, sH64, sH32, air_tw;
   GridP<F64> g64;  // operator view (kstart shift applied inside kernels)
   GridP<F32> g32;
   AirP<F64> a64;
   AirP<F32> a32;
   AcqGrid acq;
+  // complex64 airwave by k_airwave32.cu (sH32 is then transposed, air_tw its twiddles) instead
+  // of cuFFT
+  bool air_lines = false;
   // cuFFT plans of this model's airwave grid (one set per model: a plan is bound to one
   // stream at a time, and contexts may run on different host threads)
   FftPlans fft_plans;

@@ -38,7 +38,6 @@
 // 0.86 -> 0.51; 81 x 73 x 67 cells, 3 systems at 3 frequencies 0.51 -> 0.35. The pass takes
 // 60% of it, at 55% of the DRAM rate; the chain runs at 40%, bound by its steps' latency and
 // the warps that shared memory leaves room for (7 on an SM).
-#include <atomic>
 #include <type_traits>
 #include "csem_cuda.cuh"
 #include "engine.h"
@@ -479,21 +478,6 @@ __global__ void __launch_bounds__(32 * LineShape<COMP>::WARPS) k_line32(SweepP<F
 }
 
 namespace {
-
-constexpr size_t SMEM_MOST = 227 * 1024;
-
-// dynamic shared memory above 48 KB has to be asked for, once per kernel and device
-template <auto KERNEL> void allow_smem(size_t bytes)
-{
-  static std::atomic<unsigned long long> done{0};
-  if (bytes <= 48 * 1024) return;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
-  if (bit && (done.load(std::memory_order_acquire) & bit)) return;
-  if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MOST) == cudaSuccess)
-    done.fetch_or(bit, std::memory_order_release);
-}
 
 template <int COMP, bool FWD, int NS>
 void launch_pass(const SweepP<F32>& s, int sets, float2* SB, float2* SW, long sbs, const int* groups, cudaStream_t st)
