@@ -139,17 +139,26 @@ template <class P> struct SysScal {
 
 constexpr size_t SMEM_MOST = 227 * 1024;
 
-// dynamic shared memory above 48 KB has to be asked for, once per kernel and device
-template <auto KERNEL> inline void allow_smem(size_t bytes)
+// An attribute of a kernel, set once per kernel, attribute and device
+template <auto KERNEL, cudaFuncAttribute ATTR> inline void set_once(int value)
 {
   static std::atomic<unsigned long long> done{0};
-  if (bytes <= 48 * 1024) return;
   int dev = 0;
   cudaGetDevice(&dev);
   const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
   if (bit && (done.load(std::memory_order_acquire) & bit)) return;
-  if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MOST) == cudaSuccess)
-    done.fetch_or(bit, std::memory_order_release);
+  if (cudaFuncSetAttribute(KERNEL, ATTR, value) == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+}
+// dynamic shared memory above 48 KB has to be asked for
+template <auto KERNEL> inline void allow_smem(size_t bytes)
+{
+  if (bytes > 48 * 1024) set_once<KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize>((int)SMEM_MOST);
+}
+// A kernel that lives on its L1 hits asks for no more shared memory than it uses: else its CTAs
+// also go to SMs that a kernel of another stream has set to nearly all shared memory
+template <auto KERNEL> inline void keep_l1(int percent)
+{
+  set_once<KERNEL, cudaFuncAttributePreferredSharedMemoryCarveout>(percent);
 }
 
 }  // namespace csem

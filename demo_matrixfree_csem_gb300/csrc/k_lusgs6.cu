@@ -1,5 +1,4 @@
-// complex64 LU-SGS component sweeps as a pass over all points and a chain with a warp per
-// line and no barrier.
+// complex64 LU-SGS component sweeps as a pass over all points and a chain with a warp per line.
 //
 // A component sweep in linear form (k_sweep_common.cuh) is v(r, m) = B + w (gp v(r, m-1) +
 // gn v(r-1, m)) going forward, the upper neighbours going backward, on independent lines:
@@ -13,31 +12,36 @@
 // The pass: a thread per point, which forms 1/aii and w once for its frequency's systems. A
 // point's operands lie at the same offsets in every system, so they are formed once, too,
 // relative to the planes k and k-1 (k+1 for Ez), each in y or in the cap. Ex's lines are
-// i, the axis its operands are contiguous on, so 32 x 32 tiles turn in shared memory.
+// i, the axis its operands are contiguous on, so 32 x 32 tiles turn in shared memory. A thread
+// forms two points, for the loads in flight; Ey's and Ez's are of neighbouring rows j and share
+// some (11 -> 9 or 10 a point). 64 registers, for 32 warps an SM.
 //
 // The chain: a warp owns one line and works through its march in strips of 32 positions, lane t on
 // position t of the strip, over all rows of the strip before the next strip. Lane t runs t
 // rows behind lane 0, so that lane t - 1's value at its row is there, one shuffle away, when
 // it is due. Loads and stores stay together all the same: rows are copied into a queue in
-// shared memory (cp.async, 16 to 23 rows early), where lane t takes its entry t steps after
+// shared memory (cp.async, 9 to 16 rows early), where lane t takes its entry t steps after
 // lane 0 and leaves v in its place; 31 steps after lane 0 the row is complete and is stored by
 // all lanes at once. A strip's last column is kept for the left neighbours
 // of the next strip's first (edge), and the strips follow one another without draining:
 // lanes go over to the next strip one by one. Everything that does not happen at every row
-// (the strip's start, the copies and the stores) happens every 8 rows, and the 8 rows' queue
-// entries are in registers before the chain goes through them, so that a step is little more
-// than the dependence: a shuffle and four multiply-adds.
+// happens every 8 rows (4 in some shapes, launch_line), and the copies and stores are a second
+// warp's, one barrier a chunk apart from the first: with one or two lines' warps to a scheduler
+// every instruction counts towards the line's time, and a chunk's 8 rows took 700 cycles of the
+// chain and 550 of the rest in turn.
 //
-// Ex is the contiguous axis across its lines: 8 warps take 8 neighbouring lines and store
-// their rows together, 64 bytes at a time, after a barrier every 8 rows.
+// Ex is the contiguous axis across its lines: a CTA takes 8 (or 4) neighbouring lines and stores
+// their rows together, 64 bytes at a time.
 //
 // The thread-per-row pipelines (k_sweep_ex32s, k_sweep_eyz32s, lusgs_split 1) read one 16-byte
 // entry per row and lane, 20 sectors a request, and join a line's warps by barriers at every
-// step. Per application, them against this, one context: 200 x 140 x 140 cells, 48 systems
-// 23.3 -> 14.6 ms, 16 systems 8.02 -> 5.30, 3 systems 2.11 -> 1.40; 84^3 cells, 6 systems
-// 0.86 -> 0.51; 81 x 73 x 67 cells, 3 systems at 3 frequencies 0.51 -> 0.35. The pass takes
-// 60% of it, at 55% of the DRAM rate; the chain runs at 40%, bound by its steps' latency and
-// the warps that shared memory leaves room for (7 on an SM).
+// step. Per application, them, this with one warp to a line and one point to a pass's thread, and
+// this, one context: 200 x 140 x 140 cells, 48 systems 23.3, 14.6, 13.9 ms, 16 systems 8.02,
+// 5.30, 4.81, 3 systems 2.11, 1.40, 1.16; 84^3 cells, 6 systems 0.86, 0.51, 0.42; 81 x 73 x 67
+// cells, 3 systems at 3 frequencies 0.51, 0.35, 0.27. The pass takes 60% of it, at 60% of the
+// DRAM rate, bound by its loads' latency; the chain runs at 50% (large batches: 7 or 8 lines on
+// an SM by its shared memory, and its load and store unit) or is bound by its steps' latency, 640
+// cycles for 8 rows (small ones).
 #include <type_traits>
 #include "csem_cuda.cuh"
 #include "engine.h"
@@ -51,10 +55,6 @@ namespace {
 
 typedef float2 C;
 
-__device__ __forceinline__ C shfl(C v, int from)
-{
-  return make_float2(__shfl_sync(0xffffffffu, v.x, from), __shfl_sync(0xffffffffu, v.y, from));
-}
 __device__ __forceinline__ void fetch16(unsigned dst, const void* src)
 {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -62,25 +62,22 @@ __device__ __forceinline__ void fetch16(unsigned dst, const void* src)
 __device__ __forceinline__ void fetch_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void fetch_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-constexpr int CH = 8;  // rows per chunk
-// Ey, Ez: one warp to a CTA, two chunks copied ahead; Ex: 8 warps, whose shared memory leaves
-// room for one
-template <int COMP> struct LineShape {
-  static constexpr int WARPS = COMP == 0 ? 8 : 1;
-  static constexpr int AHEAD = COMP == 0 ? 1 : 2;
+// A CTA's lines (Ey, Ez: 1; Ex: 4 or 8), rows per chunk (8 or 4), chunks copied ahead
+template <int LINES, int CH> struct LineShape {
+  static constexpr int AHEAD = CH == 4 ? 3 : 2;
   static constexpr int DEPTH = 32 + CH * (1 + AHEAD);  // queue entries per lane: 32 rows in work or to be stored, and the copies
-  // a warp's queue in float2: B (and then v) [DEPTH][32], w [DEPTH][32], 4 of padding (Ex's
-  // lines on different banks)
-  static constexpr int QUEUE = 2 * DEPTH * 32 + 4;
+  // a line's queue in float2: B (and then v) [DEPTH][32], w [DEPTH][32], padding (Ex's lines on
+  // different banks)
+  static constexpr int QUEUE = 2 * DEPTH * 32 + (LINES > 1 ? 16 / LINES : 0);
 };
 constexpr unsigned QE = 256;  // bytes from a lane's queue entry to its next
 
 // shared memory: queues, edge columns float2 [warps][Rp + 32], row couplings float [32 + Rp]
 // (the first 32: the last rows of the strip before)
-template <int COMP> inline size_t line_smem(int R)
+template <int LINES, int CH> inline size_t line_smem(int R)
 {
   const size_t Rp = line_steps(R);
-  return LineShape<COMP>::WARPS * (LineShape<COMP>::QUEUE * 8 + (Rp + 32) * 8) + (Rp + 32) * 4;
+  return LINES * (LineShape<LINES, CH>::QUEUE * 8 + (Rp + 32) * 8) + (Rp + 32) * 4;
 }
 
 // A point's coupling to the other two components and its own not-yet-swept neighbours, at
@@ -125,97 +122,143 @@ __device__ __forceinline__ long plane(const SweepP<F32>& s, int c, int k, bool u
   return (up ? g.lEx + g.lEy : s.capEx + s.capEy) + kk * (g.n1 + 1) * (g.n2 + 1);
 }
 
-constexpr int PASS_WARPS = 4;
+constexpr int PASS_WARPS = 2;
+// Percent of an SM's 228 KB that the passes leave for shared memory (Ex's uses 34 KB). With the
+// chains' setting (all of it) the passes' loads miss L1: 16 systems 4.81 -> 6.38 ms an
+// application, and 6.04 where two contexts' applications overlap; so 4.81 and 4.60
+constexpr int PASS_SMEM = 20;
 
 }  // namespace
 
-// Ey and Ez: a warp per strip of a row, PASS_WARPS neighbouring j. grid (strips x groups, j, k)
+// Ey and Ez: a warp per strip of a pair of rows j, PASS_WARPS pairs. grid (strips x groups, pairs, k)
 template <int COMP, bool FWD, int NS>
-__global__ void __launch_bounds__(32 * PASS_WARPS)
+__global__ void __launch_bounds__(32 * PASS_WARPS, 16)
     k_line_pass(SweepP<F32> s, float2* SB, float2* SW, long sbs, const int* groups)
 {
   const GridP<F32>& g = s.g;
   const int n1 = g.n1, n2 = g.n2, nK = s.nK, L1 = n1 + 1;
   const int M = n1 - 1, R = COMP == 1 ? nK - 1 : n2 - 1, S = line_strips(M), Rp = line_steps(R);
   const int grp = blockIdx.x / S, strip = blockIdx.x - grp * S;
-  const int lane = threadIdx.x & 31, j = blockIdx.y * PASS_WARPS + (threadIdx.x >> 5) + (COMP == 2 ? 1 : 0);
+  const int lane = threadIdx.x & 31, j0 = 2 * (blockIdx.y * PASS_WARPS + (threadIdx.x >> 5)) + (COMP == 2 ? 1 : 0);
   const int k = blockIdx.z + (COMP == 1 ? 1 : 0);
   const int p = strip * 32 + lane, i = FWD ? min(1 + p, M) : max(M - p, 1);
   const Members<NS> mem(s, groups, grp);
   const SysScal<F32> sc = s.scal[mem.sys_of(0)];
-  if (j >= n2) return;
-  const bool on = p < M;  // (lanes past the last position form position M again, and store nothing)
+  if (j0 >= n2) return;
+  // lanes past the last position form position M again, and a last row without a pair is formed
+  // twice; neither is stored
+  const bool on = p < M, pair = j0 + 1 < n2;
   // Ey: row axis Z (k), line axis Y (j); Ez: row axis Y (j), line axis Z (k)
-  const Ax<F32> Rw = COMP == 1 ? axis<F32>(g.d3, g.d3s, g.r3, g.r3s, k) : axis<F32>(g.d2, g.d2s, g.r2, g.r2s, j);
-  const Ax<F32> LA = COMP == 1 ? axis_at<F32>(g.d2, g.d2s, g.r2, g.r2s, j) : axis_at<F32>(g.d3, g.d3s, g.r3, g.r3s, k);
   const Ax<F32> X = axis<F32>(g.d1, g.d1s, g.r1, g.r1s, i);
-  const float gg = (X.rs + X.rsm) * X.r + (Rw.rs + Rw.rsm) * Rw.r;  // geo(Z, X) / geo(X, Y)
-  const float ydd = COMP == 1 ? LA.d : Rw.d, zdd = COMP == 1 ? Rw.d : LA.d;
-  const float sg = ro(COMP == 1 ? g.s22 + ix2(n1, n2, k, j, i) : g.s33 + ix3(n1, n2, k, j, i));
-  const Coef32 cf = lin_coef(sc, g.fvm, gg, sg, X.ds * ydd * zdd);
-  const size_t e = line_entry(S, Rp, COMP == 1 ? j : k, p, COMP == 1 ? (FWD ? k - 1 : R - k) : (FWD ? j - 1 : R - j));
-  if (on) SW[(size_t)grp * sbs + e] = cf.w;
+  Coef32 cf[2];
+  float rr[2], lrs[2], kr[2];  // the row's 1/d, the line's 1/ds, the coupling to the row below
+  size_t e[2];
+#pragma unroll
+  for (int a = 0; a < 2; a++) {
+    const int j = min(j0 + a, n2 - 1);
+    const Ax<F32> Rw = COMP == 1 ? axis<F32>(g.d3, g.d3s, g.r3, g.r3s, k) : axis<F32>(g.d2, g.d2s, g.r2, g.r2s, j);
+    const Ax<F32> LA = COMP == 1 ? axis_at<F32>(g.d2, g.d2s, g.r2, g.r2s, j) : axis_at<F32>(g.d3, g.d3s, g.r3, g.r3s, k);
+    const float gg = (X.rs + X.rsm) * X.r + (Rw.rs + Rw.rsm) * Rw.r;  // geo(Z, X) / geo(X, Y)
+    const float ydd = COMP == 1 ? LA.d : Rw.d, zdd = COMP == 1 ? Rw.d : LA.d;
+    const float sg = ro(COMP == 1 ? g.s22 + ix2(n1, n2, k, j, i) : g.s33 + ix3(n1, n2, k, j, i));
+    cf[a] = lin_coef(sc, g.fvm, gg, sg, X.ds * ydd * zdd);
+    rr[a] = Rw.r;
+    lrs[a] = -LA.rs;
+    kr[a] = Rw.r * Rw.rsm;
+    e[a] = line_entry(S, Rp, COMP == 1 ? j : k, p, COMP == 1 ? (FWD ? k - 1 : R - k) : (FWD ? j - 1 : R - j));
+    if (on && (a == 0 || pair)) SW[(size_t)grp * sbs + e[a]] = cf[a].w;
+  }
   const int kB = COMP == 1 ? k - 1 : k + 1;
   const bool upA = k >= s.vshift, upB = kB >= s.vshift;
-  // Ex and the third component either side of the line, own old values on the lower side
-  const unsigned xb = 8u * (unsigned)(plane(s, 0, k, upA) + (long)j * n1 + i);
-  const unsigned xa = COMP == 1 ? xb + 8u * n1 : 8u * (unsigned)(plane(s, 0, kB, upB) + (long)j * n1 + i);
-  unsigned ya, yb, yc, yd;  // upper and lower side of the line, at the row and at the row below
+  // rows of Ex: Ey j0, j0 + 1, j0 + 2 of plane k; Ez j0, j0 + 1 of planes k and kB. Rows of the
+  // third component, both planes: Ey's Ez j0, j0 + 1, j0 + 2; Ez's Ey j0 - 1, j0, j0 + 1
+  unsigned xo[4], yo[6], own[2], low[2];
+  const unsigned px = 8u * (unsigned)(plane(s, 0, k, upA) + i), py = 8u * (unsigned)(plane(s, 3 - COMP, k, upA) + i);
+  const unsigned qy = 8u * (unsigned)(plane(s, 3 - COMP, kB, upB) + i), po = 8u * (unsigned)(plane(s, COMP, k, upA) + i);
   if (COMP == 1) {
-    yb = 8u * (unsigned)(plane(s, 2, k, upA) + (long)j * L1 + i), ya = yb + 8u * L1;
-    yd = 8u * (unsigned)(plane(s, 2, kB, upB) + (long)j * L1 + i), yc = yd + 8u * L1;
+    const unsigned ql = 8u * (unsigned)(plane(s, 1, kB, upB) + i);
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      const unsigned j = min(j0 + r, n2);
+      xo[r] = px + 8u * n1 * j;
+      yo[r] = py + 8u * L1 * j;
+      yo[3 + r] = qy + 8u * L1 * j;
+    }
+#pragma unroll
+    for (int a = 0; a < 2; a++) {
+      const unsigned j = min(j0 + a, n2 - 1);
+      own[a] = po + 8u * L1 * j;
+      low[a] = ql + 8u * L1 * j;
+    }
   } else {
-    yb = 8u * (unsigned)(plane(s, 1, k, upA) + (long)j * L1 + i), yd = yb - 8u * L1;
-    ya = 8u * (unsigned)(plane(s, 1, kB, upB) + (long)j * L1 + i), yc = ya - 8u * L1;
+    const unsigned qx = 8u * (unsigned)(plane(s, 0, kB, upB) + i);
+#pragma unroll
+    for (int a = 0; a < 2; a++) {
+      const unsigned j = min(j0 + a, n2 - 1);
+      xo[a] = qx + 8u * n1 * j;
+      xo[2 + a] = px + 8u * n1 * j;
+      own[a] = po + 8u * L1 * j;
+      low[a] = own[a] - 8u * L1;
+    }
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      const unsigned j = min(j0 + r, n2) - 1;
+      yo[r] = py + 8u * L1 * j;
+      yo[3 + r] = qy + 8u * L1 * j;
+    }
   }
-  const unsigned own = 8u * (unsigned)(plane(s, COMP, k, upA) + (long)j * L1 + i);
-  const unsigned low = COMP == 1 ? 8u * (unsigned)(plane(s, 1, kB, upB) + (long)j * L1 + i) : own - 8u * L1;
-  const float km = X.r * X.rsm, kr = Rw.r * Rw.rsm;
+  const float km = X.r * X.rsm;
   const C z = make_float2(0.f, 0.f);
-  float2* out = SB + e;
   struct Vals {
-    C b, xa, xb, xc, xd, ya, yb, yc, yd, o, lo;
+    C b[2], x[4], xm[4], y[6], o[2], lo[2];
   };
   auto load = [&](int q) {
     const Bases m = bases(s, mem.slot_of(q), mem.sys_of(q), upA, upB);
-    const char* const xA = COMP == 1 ? m.A : m.B;
     Vals v;
-    v.b = upA ? at(m.x, own) : z;
-    v.xa = at(xA, xa), v.xb = at(m.A, xb), v.xc = at(xA, xa - 8), v.xd = at(m.A, xb - 8);
-    if (COMP == 2 || !FWD) {
-      v.ya = at(COMP == 1 ? m.A : m.B, ya), v.yb = at(m.A, yb);
-      v.yc = at(m.B, yc), v.yd = at(COMP == 1 ? m.B : m.A, yd);
+#pragma unroll
+    for (int a = 0; a < 2; a++) v.b[a] = upA ? at(m.x, own[a]) : z;
+#pragma unroll
+    for (int r = 0; r < (COMP == 1 ? 3 : 4); r++) {
+      const char* const x = COMP == 2 && r < 2 ? m.B : m.A;
+      v.x[r] = at(x, xo[r]), v.xm[r] = at(x, xo[r] - 8);
     }
-    if (!FWD) v.o = at(m.A, own - 8), v.lo = at(COMP == 1 ? m.B : m.A, low);
+    if (COMP == 2 || !FWD) {
+#pragma unroll
+      for (int r = 0; r < 6; r++) v.y[r] = at(r < 3 ? m.A : m.B, yo[r]);
+    }
+    if (!FWD) {
+#pragma unroll
+      for (int a = 0; a < 2; a++) v.o[a] = at(m.A, own[a] - 8), v.lo[a] = at(COMP == 1 ? m.B : m.A, low[a]);
+    }
     return v;
   };
   auto form = [&](int q, const Vals& v) {
-    const C dx = sub32(sub32(v.xa, v.xb), sub32(v.xc, v.xd));
-    // Ey: Y.rs (Z.r dEz + X.r dEx); Ez: Z.rs (X.r dEx + Y.r dEy)
-    C acc = scl32(X.r, dx);
-    if (COMP == 2 || !FWD) {
-      const C dy = sub32(sub32(v.ya, v.yb), sub32(v.yc, v.yd));
-      acc = make_float2(acc.x + Rw.r * dy.x, acc.y + Rw.r * dy.y);
+    float2* const out = SB + (size_t)mem.slot_of(q) * sbs;
+#pragma unroll
+    for (int a = 0; a < 2; a++) {
+      const int u = COMP == 1 ? a + 1 : a, l = COMP == 1 ? a : a + 2;  // Ex on the upper and the lower side
+      const C dx = sub32(sub32(v.x[u], v.x[l]), sub32(v.xm[u], v.xm[l]));
+      // Ey: Y.rs (Z.r dEz + X.r dEx); Ez: Z.rs (X.r dEx + Y.r dEy)
+      C acc = scl32(X.r, dx);
+      if (COMP == 2 || !FWD) {
+        const C dy = COMP == 1 ? sub32(sub32(v.y[a + 1], v.y[a]), sub32(v.y[a + 4], v.y[a + 3]))
+                               : sub32(sub32(v.y[a + 4], v.y[a + 1]), sub32(v.y[a + 3], v.y[a]));
+        acc = make_float2(acc.x + rr[a] * dy.x, acc.y + rr[a] * dy.y);
+      }
+      C kc = scl32(lrs[a], acc);
+      if (!FWD) kc = make_float2(kc.x + (km * v.o[a].x + kr[a] * v.lo[a].x), kc.y + (km * v.o[a].y + kr[a] * v.lo[a].y));
+      const C B = lin_B(cf[a], g.fvm, v.b[a], kc);
+      if (on && (a == 0 || pair)) out[e[a]] = B;
     }
-    C kc = scl32(-LA.rs, acc);
-    if (!FWD) kc = make_float2(kc.x + (km * v.o.x + kr * v.lo.x), kc.y + (km * v.o.y + kr * v.lo.y));
-    const C B = lin_B(cf, g.fvm, v.b, kc);
-    const int slot = mem.slot_of(q);
-    if (on) out[(size_t)slot * sbs] = B;
   };
-  int q = 0;
-  for (; q + 1 < mem.n; q += 2) {  // two systems' loads in flight
-    const Vals v = load(q), u = load(q + 1);
-    form(q, v);
-    form(q + 1, u);
-  }
-  if (q < mem.n) form(q, load(q));
+#pragma unroll 1
+  for (int q = 0; q < mem.n; q++) form(q, load(q));
 }
 
 // Ex: a CTA forms 32 i x a strip's 32 positions j, along i, and stores them along j.
 // grid (i tiles x groups, strips, k)
 template <bool FWD, int NS>
-__global__ void __launch_bounds__(512) k_line_pass_ex(SweepP<F32> s, float2* SB, float2* SW, long sbs, int nti, const int* groups)
+__global__ void __launch_bounds__(512, 2) k_line_pass_ex(SweepP<F32> s, float2* SB, float2* SW, long sbs, int nti, const int* groups)
 {
   __shared__ C tiles[2][32][33];  // one is written while the other's values go out
   const GridP<F32>& g = s.g;
@@ -245,14 +288,14 @@ __global__ void __launch_bounds__(512) k_line_pass_ex(SweepP<F32> s, float2* SB,
     oy[a] = 8u * (unsigned)(plane(s, 1, k, upA) + (long)j * L1 + i);
     oz[a] = 8u * (unsigned)(plane(s, 2, k, upA) + (long)j * L1 + i);
     ozm[a] = 8u * (unsigned)(plane(s, 2, k - 1, upB) + (long)j * L1 + i);
-    tiles[1][ty + 16 * a][tx] = cf[a].w;
+    tiles[1][tx][ty + 16 * a] = cf[a].w;
   }
   const size_t e0 = line_entry(S, Rp, i0 + ty, 32 * blockIdx.y + tx, FWD ? k - 1 : R - k), e1 = line_entry(S, Rp, 16, 0, 0);
   const bool w0 = i0 + ty < n1, w1 = i0 + ty + 16 < n1;
   auto turn = [&](C(*tile)[33], C* out) {
     __syncthreads();
-    if (w0) out[e0] = tile[tx][ty];
-    if (w1) out[e0 + e1] = tile[tx][ty + 16];
+    if (w0) out[e0] = tile[ty][tx];
+    if (w1) out[e0 + e1] = tile[ty + 16][tx];
   };
   turn(tiles[1], SW + (size_t)grp * sbs);
   const C z = make_float2(0.f, 0.f);
@@ -286,19 +329,19 @@ __global__ void __launch_bounds__(512) k_line_pass_ex(SweepP<F32> s, float2* SB,
         const C cross = scl32(xrs, make_float2(yr[a] * dy.x + Z.r * dz.x, yr[a] * dy.y + Z.r * dz.y));
         kc = sub32(make_float2(kj[a] * v[a].ej.x + kz * v[a].ek.x, kj[a] * v[a].ej.y + kz * v[a].ek.y), cross);
       }
-      tile[ty + 16 * a][tx] = lin_B(cf[a], g.fvm, v[a].b, kc);
+      tile[tx][ty + 16 * a] = lin_B(cf[a], g.fvm, v[a].b, kc);
     }
     if (q + 1 < mem.n) load(q + 1);  // in flight while this system's tile turns
     turn(tile, SB + (size_t)mem.slot_of(q) * sbs);
   }
 }
 
-template <int COMP, bool FWD>
-__global__ void __launch_bounds__(32 * LineShape<COMP>::WARPS) k_line32(SweepP<F32> s, const float2* SB, const float2* SW,
+template <int COMP, bool FWD, int LINES, int CH>
+__global__ void __launch_bounds__(64 * LINES) k_line32(SweepP<F32> s, const float2* SB, const float2* SW,
                                                                         long sbs, const int* group_of, int groups_per_slot)
 {
-  constexpr int WARPS = LineShape<COMP>::WARPS, AHEAD = LineShape<COMP>::AHEAD, DEPTH = LineShape<COMP>::DEPTH,
-                QUEUE = LineShape<COMP>::QUEUE;
+  typedef LineShape<LINES, CH> Shape;
+  constexpr int AHEAD = Shape::AHEAD, DEPTH = Shape::DEPTH, QUEUE = Shape::QUEUE;
   constexpr unsigned QW = DEPTH * QE;  // bytes from a B to its w
   extern __shared__ float2 smem[];
   const GridP<F32>& g = s.g;
@@ -308,10 +351,11 @@ __global__ void __launch_bounds__(32 * LineShape<COMP>::WARPS) k_line32(SweepP<F
   const int M = COMP == 0 ? n2 - 1 : n1 - 1;  // march positions 1..M
   const int Rp = line_steps(R);
   const int S = (M + 31) / 32;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % LINES;
+  const bool mover = threadIdx.x >= 32 * LINES;  // a line's second warp: its copies and stores
   const int slot = blockIdx.x / groups_per_slot;
-  const int line0 = (blockIdx.x - slot * groups_per_slot) * WARPS;
-  const int line = WARPS > 1 ? min(line0 + warp, nlines - 1) : line0;  // (a CTA's warps stay together)
+  const int line0 = (blockIdx.x - slot * groups_per_slot) * LINES;
+  const int line = LINES > 1 ? min(line0 + warp, nlines - 1) : line0;  // (a CTA's warps stay together)
   const int sys = s.sys_list ? s.sys_list[slot] : slot;
   const View<F32> V = view_of<F32>(s, slot, sys);
   const C z = make_float2(0.f, 0.f);
@@ -319,10 +363,10 @@ __global__ void __launch_bounds__(32 * LineShape<COMP>::WARPS) k_line32(SweepP<F
   auto row_of = [&](int rho) { return FWD ? 1 + rho : R - rho; };
   auto col = [&](int st) { return FWD ? 1 + 32 * st + lane : M - 32 * st - lane; };
 
-  C* const edge = smem + WARPS * QUEUE + warp * (Rp + 32);
-  float* const rowgn = (float*)(smem + WARPS * QUEUE + WARPS * (Rp + 32));
+  C* const edge = smem + LINES * QUEUE + warp * (Rp + 32);
+  float* const rowgn = (float*)(smem + LINES * QUEUE + LINES * (Rp + 32));
   // what couples a step's row to the row before
-  for (int q = threadIdx.x; q < 32 + Rp; q += 32 * WARPS) {
+  for (int q = threadIdx.x; q < 32 + Rp; q += 64 * LINES) {
     const int rho = q < 32 ? q - 32 + Rp : q - 32;
     float gn = 0.f;
     if (rho < R) {
@@ -332,7 +376,6 @@ __global__ void __launch_bounds__(32 * LineShape<COMP>::WARPS) k_line32(SweepP<F
     rowgn[q] = gn;
   }
   for (int q = lane; q < Rp + 32; q += 32) edge[q] = z;
-  __syncthreads();
 
   char* const queue = (char*)(smem + warp * QUEUE + lane);
 
@@ -383,20 +426,21 @@ __global__ void __launch_bounds__(32 * LineShape<COMP>::WARPS) k_line32(SweepP<F
       B[u] = *(const C*)(queue + q[u]);
       w[u] = *(const C*)(queue + q[u] + QW);
       gn[u] = gl[cf + u];
-      le[u] = edge[cf + u + 31];  // the strip before, at lane 0's row
+      le[u] = z;
+      if (lane == 0) le[u] = edge[cf + u + 31];  // the strip before, at lane 0's row
     }
 #pragma unroll
     for (int u = 0; u < CH; u++) {
-      C left = shfl(v, lane - 1);
-      left.x = lane == 0 ? le[u].x : left.x;
-      left.y = lane == 0 ? le[u].y : left.y;
+      const C left = make_float2(__shfl_up_sync(0xffffffffu, v.x, 1), __shfl_up_sync(0xffffffffu, v.y, 1));
       if constexpr (starting.value) {
         const bool now = cf + u == lane;
         gp = now ? gpn : gp;
         v.x = now ? 0.f : v.x;
         v.y = now ? 0.f : v.y;
       }
-      const C t = make_float2(gp * left.x + gn[u] * v.x, gp * left.y + gn[u] * v.y);
+      const float gs = lane == 0 ? 0.f : gp;
+      const C d = make_float2(gp * le[u].x + gn[u] * v.x, gp * le[u].y + gn[u] * v.y);
+      const C t = make_float2(d.x + gs * left.x, d.y + gs * left.y);
       v = make_float2(B[u].x + w[u].x * t.x - w[u].y * t.y, B[u].y + w[u].x * t.y + w[u].y * t.x);
       B[u] = v;
     }
@@ -417,7 +461,7 @@ __global__ void __launch_bounds__(32 * LineShape<COMP>::WARPS) k_line32(SweepP<F
   const long so = COMP == 0 ? (long)n1 * (n2 + 1) : (COMP == 1 ? (long)L1 * n2 : L1);
   C* const oU = COMP == 2 ? V.row(2, line, 0) : V.row(COMP, k0, COMP == 1 ? line : 0) - k0 * so;
   C* const oL = COMP == 2 || !V.CAP[COMP] ? oU : V.CAP[COMP] + (COMP == 1 ? (long)line * L1 : 0);
-  int sw = 0, rw = -32;
+  int sw = 0, rw = -32;  // strip and first row
   unsigned wq = (DEPTH - 32) * QE;  // their first entry
   auto store = [&]() {
     if (rw >= 0 && rw < R) {
@@ -434,15 +478,15 @@ __global__ void __launch_bounds__(32 * LineShape<COMP>::WARPS) k_line32(SweepP<F
           }
         }
       } else {
-        // this warp's row of the chunk: 4 positions of 8 lines at a time
-        const int i = line0 + (lane & 7), r = row_of(rw + warp);
-        if (rw + warp < R && i < n1) {
-          C* const out = (r >= k0 ? oU : oL) + r * so + i;
-          const char* const in = (const char*)(smem + (lane & 7) * QUEUE) + wq + warp * QE;
+        // 32 / LINES positions of all lines for each warp
+        const int t = (32 * warp + lane) / LINES, l = lane % LINES, pos = 32 * sw + t, i = line0 + l;
+        if (pos < M && i < n1) {
+          const long o = (long)(FWD ? 1 + pos : M - pos) * n1 + i;
+          const char* const in = (const char*)(smem + l * QUEUE + t) + wq;
 #pragma unroll
-          for (int a = 0; a < 8; a++) {
-            const int t = a * 4 + (lane >> 3), m = FWD ? 1 + 32 * sw + t : M - 32 * sw - t;
-            if (m >= 1 && m <= M) out[(long)m * n1] = *(const C*)(in + t * 8);
+          for (int u = 0; u < CH; u++) {
+            const int r = row_of(rw + u);
+            if (rw + u < R) ((r >= k0 ? oU : oL) + r * so)[o] = *(const C*)(in + u * QE);
           }
         }
       }
@@ -455,26 +499,37 @@ __global__ void __launch_bounds__(32 * LineShape<COMP>::WARPS) k_line32(SweepP<F
     wq = wq + CH * QE == DEPTH * QE ? 0 : wq + CH * QE;
   };
 
-#pragma unroll
-  for (int q = 0; q < AHEAD; q++) copy();
+  // Chunk c: the line's warp goes through it, while the other stores the rows that chunk c - 1
+  // completed, copies chunk c + AHEAD into their entries and waits for chunk c + 1's.
   const int chunks = ((S - 1) * Rp + R + 32 + CH - 1) / CH;
-  for (int c = 0; c < chunks; c++) {
-    if (cf == 0) {
-      gpn = gpl;
-      gpl = coupling(++sf);
-    }
+  if (mover) {
+#pragma unroll
+    for (int q = 0; q < AHEAD; q++) copy();
     fetch_wait<AHEAD - 1>();
-    __syncwarp();  // the other lanes' copies are there, too
-    copy();
-    if (cf < 32) chain(std::true_type(), c < 4);
-    else chain(std::false_type(), false);
-    cf = cf + CH == Rp ? 0 : cf + CH;
-    if (WARPS > 1) __syncthreads();  // every line has its part of the rows
-    else __syncwarp();               // edge
+    __syncthreads();
+    for (int c = 0; c < chunks; c++) {
+      if (c > 0) store();
+      if (LINES > 1) asm volatile("bar.sync 1, %0;" ::"n"(32 * LINES) : "memory");
+      else __syncwarp();
+      copy();
+      fetch_wait<AHEAD - 1>();
+      __syncthreads();
+    }
     store();
-    if (WARPS > 1) __syncthreads();  // before the next copies take the entries
+    fetch_wait<0>();
+  } else {
+    __syncthreads();
+    for (int c = 0; c < chunks; c++) {
+      if (cf == 0) {
+        gpn = gpl;
+        gpl = coupling(++sf);
+      }
+      if (cf < 32) chain(std::true_type(), c * CH < 32);
+      else chain(std::false_type(), false);
+      cf = cf + CH == Rp ? 0 : cf + CH;
+      __syncthreads();
+    }
   }
-  fetch_wait<0>();
 }
 
 namespace {
@@ -484,12 +539,14 @@ void launch_pass(const SweepP<F32>& s, int sets, float2* SB, float2* SW, long sb
 {
   const int n1 = s.g.n1, n2 = s.g.n2, nK = s.nK;
   if constexpr (COMP == 0) {
-    const int nti = (n1 + 31) / 32;
+    const int nti = (n1 + 32 - 1) / 32;
     dim3 grd((unsigned)(nti * sets), (unsigned)line_strips(n2 - 1), (unsigned)(nK - 1));
+    keep_l1<k_line_pass_ex<FWD, NS>>(PASS_SMEM);
     count_launch(), k_line_pass_ex<FWD, NS><<<grd, 512, 0, st>>>(s, SB, SW, sbs, nti, groups);
   } else {
     const int js = COMP == 1 ? n2 : n2 - 1, ks = COMP == 1 ? nK - 1 : nK;
-    dim3 grd((unsigned)(line_strips(n1 - 1) * sets), (unsigned)((js + PASS_WARPS - 1) / PASS_WARPS), (unsigned)ks);
+    dim3 grd((unsigned)(line_strips(n1 - 1) * sets), (unsigned)((js + 2 * PASS_WARPS - 1) / (2 * PASS_WARPS)), (unsigned)ks);
+    keep_l1<k_line_pass<COMP, FWD, NS>>(PASS_SMEM);
     count_launch(), k_line_pass<COMP, FWD, NS><<<grd, 32 * PASS_WARPS, 0, st>>>(s, SB, SW, sbs, groups);
   }
 }
@@ -501,16 +558,38 @@ void launch_passes(const SweepP<F32>& s, int nslot, float2* SB, float2* SW, long
   else launch_pass<COMP, FWD, 1>(s, nslot, SB, SW, sbs, nullptr, st);
 }
 
+template <int COMP, bool FWD, int LINES, int CH>
+void launch_line_of(const SweepP<F32>& s, int nslot, const float2* SB, const float2* SW, long sbs, const int* group_of,
+                    cudaStream_t st)
+{
+  const int R = COMP == 2 ? s.g.n2 - 1 : s.nK - 1, nlines = COMP == 0 ? s.g.n1 : (COMP == 1 ? s.g.n2 : s.nK);
+  const int gps = (nlines + LINES - 1) / LINES;
+  const size_t sm = line_smem<LINES, CH>(R);
+  const auto kernel = k_line32<COMP, FWD, LINES, CH>;
+  allow_smem<k_line32<COMP, FWD, LINES, CH>>(sm);
+  count_launch(), kernel<<<(unsigned)((long)gps * nslot), 64 * LINES, sm, st>>>(s, SB, SW, sbs, group_of, gps);
+}
 template <int COMP, bool FWD>
 void launch_line(const SweepP<F32>& s, int nslot, const float2* SB, const float2* SW, long sbs, const int* group_of,
                  cudaStream_t st)
 {
-  constexpr int W = LineShape<COMP>::WARPS;
-  const int R = COMP == 2 ? s.g.n2 - 1 : s.nK - 1, nlines = COMP == 0 ? s.g.n1 : (COMP == 1 ? s.g.n2 : s.nK);
-  const int gps = (nlines + W - 1) / W;
-  const size_t sm = line_smem<COMP>(R);
-  allow_smem<k_line32<COMP, FWD>>(sm);
-  count_launch(), k_line32<COMP, FWD><<<(unsigned)((long)gps * nslot), 32 * W, sm, st>>>(s, SB, SW, sbs, group_of, gps);
+  const long sms = sm_count();
+  if constexpr (COMP != 0) {
+    // chunks of 4 rows cost 3% more than chunks of 8, but 8 lines fit an SM instead of 7: taken
+    // where that saves one of few rounds of the SMs (an application, 200 x 140 x 140 cells: 8
+    // systems 2.71 -> 2.55 ms, 16 4.81 -> 4.70, 24 7.09 -> 7.00, 32 9.37 -> 9.34; 48, from 7
+    // rounds to 6, 13.88 -> 13.97)
+    const long lines = (long)(COMP == 1 ? s.g.n2 : s.nK) * nslot;
+    const long rounds7 = (lines + 7 * sms - 1) / (7 * sms), rounds8 = (lines + 8 * sms - 1) / (8 * sms);
+    if (rounds8 < rounds7 && rounds7 <= 5) launch_line_of<COMP, FWD, 1, 4>(s, nslot, SB, SW, sbs, group_of, st);
+    else launch_line_of<COMP, FWD, 1, 8>(s, nslot, SB, SW, sbs, group_of, st);
+  } else {
+    // 8 lines to a CTA fill an SM and store 64 bytes at a time, but share its load and store unit:
+    // 4 where every CTA of 4 has an SM of its own (an application, 200 x 140 x 140 cells, 8
+    // against 4 lines: 2 systems 1.05 and 0.97 ms, 3 1.24 and 1.18, 4 (200 CTAs) 1.44 and 1.49)
+    if ((long)((s.g.n1 + 3) / 4) * nslot <= sms) launch_line_of<0, FWD, 4, 8>(s, nslot, SB, SW, sbs, group_of, st);
+    else launch_line_of<0, FWD, 8, 4>(s, nslot, SB, SW, sbs, group_of, st);
+  }
 }
 
 }  // namespace
@@ -520,8 +599,7 @@ void launch_line(const SweepP<F32>& s, int nslot, const float2* SB, const float2
 bool sweep_line_fits(int n1, int n2, int nK)
 {
   const double most = 8.0 * 3.0 * (n1 + 1.0) * (n2 + 1.0) * (nK + 1.0);
-  return most < 4294967296.0 && n1 >= 2 && n2 >= 2 && nK >= 2 && line_smem<0>(nK - 1) <= SMEM_MOST && line_smem<1>(nK - 1) <= SMEM_MOST &&
-         line_smem<2>(n2 - 1) <= SMEM_MOST;
+  return most < 4294967296.0 && n1 >= 2 && n2 >= 2 && nK >= 2 && line_smem<8, 4>(nK - 1) <= SMEM_MOST && line_smem<1, 8>(n2 - 1) <= SMEM_MOST;
 }
 
 void launch_line_pass(const SweepP<F32>& s, int comp, bool fwd, int nslot, float2* SB, float2* SW, long sbs,

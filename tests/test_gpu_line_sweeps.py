@@ -53,3 +53,15 @@ def test_groups_of_any_size_give_each_system_its_own_bits(gpu, tmp_path, counts)
     got = _lusgs_batch(ctx, freqs, X)
     for q, f in enumerate(freqs):
         assert np.array_equal(got[q], _lusgs_batch(ctx, [f], X[q:q + 1])[0])
+
+
+@pytest.mark.parametrize("shape", [(29, 3, 30, 2), (3, 30, 29, 2)], ids=["29x3x30x2", "3x30x29x2"])
+def test_large_batches_give_each_system_its_own_bits(gpu, tmp_path, shape):
+    """33 systems: more lines than 7 on each of 152 SMs (chunks of 4 rows), and more of Ex's CTAs
+    than SMs (8 lines to a CTA); a system alone takes the other shapes."""
+    ctx, _ = _setup(tmp_path, 95, shape, 1, 0)
+    freqs = [(0.5, 1.0, 0.25)[q % 3] for q in range(33)]
+    X = np.stack([probe(ctx.lE, 60 + q) for q in range(len(freqs))])
+    got = _lusgs_batch(ctx, freqs, X)
+    for q in (0, 1, 16, 31, 32):
+        assert np.array_equal(got[q], _lusgs_batch(ctx, freqs[q:q + 1], X[q:q + 1])[0])
