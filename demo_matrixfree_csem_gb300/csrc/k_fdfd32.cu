@@ -18,6 +18,7 @@
 // loads and 64-bit addresses); tiles 4 and 16 rows high 850 and 1070 us. Of about 230
 // instructions a warp and plane 70 are arithmetic; registers (72, for three CTAs of 8 rows
 // on an SM) limit the loads in flight.
+#include <type_traits>
 #include "csem_cuda.cuh"
 #include "engine.h"
 #include "k_dot_common.cuh"
@@ -222,10 +223,15 @@ void launch_by(const GridP<F32>& g, const SysScal<F32>* scal, const C* X, C* Y, 
   if (by != 4 && by != 16) by = 8;
   const FdfdShape f = fdfd_shape(g.n1, g.n2, g.n3, nsys, by, ctas_per_sm, FDFD32_TILE);
   dim3 blk(32, by + 1), grd(f.gx, f.gy, nsys * f.nkc);
-  count_launch();
-  if (by == 4) k_fdfd32<4, EPI><<<grd, blk, 0, st>>>(g, scal, X, Y, ghx, ghy, f.kchunk, f.nkc, sys_list, E, part);
-  else if (by == 16) k_fdfd32<16, EPI><<<grd, blk, 0, st>>>(g, scal, X, Y, ghx, ghy, f.kchunk, f.nkc, sys_list, E, part);
-  else k_fdfd32<8, EPI><<<grd, blk, 0, st>>>(g, scal, X, Y, ghx, ghy, f.kchunk, f.nkc, sys_list, E, part);
+  auto go = [&](auto tile) {
+    constexpr int BY = decltype(tile)::value;
+    // of 228 KB; three CTAs use 28 (16 systems' operators on three streams: 1094 -> 921 us each)
+    keep_l1<k_fdfd32<BY, EPI>>(20);
+    count_launch(), k_fdfd32<BY, EPI><<<grd, blk, 0, st>>>(g, scal, X, Y, ghx, ghy, f.kchunk, f.nkc, sys_list, E, part);
+  };
+  if (by == 4) go(std::integral_constant<int, 4>());
+  else if (by == 16) go(std::integral_constant<int, 16>());
+  else go(std::integral_constant<int, 8>());
 }
 
 }  // namespace
