@@ -485,13 +485,17 @@ void Ops<P>::apply_lusgs(const C* X, C* Y, int nslot, const int* sys_list, const
     s.capEx = (long)nb * n1 * (n2 + 1);
     s.capEy = (long)nb * (n1 + 1) * n2;
     s.capE = s.capEx + s.capEy + (long)nb * (n1 + 1) * (n2 + 1);
-    if (!bounds_zero) CSEM_CUDA_TRY(cudaMemsetAsync(cap.p, 0, sizeof(C) * (size_t)s.capE * nslot, st));
   }
-  if (!bounds_zero) zero(Y, m->lE, nslot, sys_list);
+  const bool lines = line_fits();
+  if (!bounds_zero && !lines) {
+    if (s.CAP) CSEM_CUDA_TRY(cudaMemsetAsync(cap.p, 0, sizeof(C) * (size_t)s.capE * nslot, st));
+    zero(Y, m->lE, nslot, sys_list);
+  }
   if constexpr (!P::exact) {
     // the systems of one frequency grouped, where the slots are not numbered within halves
     const bool g16 = grp && grp->ns == SPLIT_GROUP && grp->n > 0 && grp->nA == 0;
-    if (line_fits()) {
+    if (lines) {
+      if (!bounds_zero) launch_line_bounds(s, nslot, st);
       const long sbs = sweep_split_scratch(n1, n2, s.nK);
       if (sb.bytes < sizeof(float4) * (size_t)sbs * nmax) sb.alloc(sizeof(float4) * (size_t)sbs * nmax);
       float2 *B = sb.as<float2>(), *W = B + (size_t)nslot * sbs;

@@ -9,7 +9,7 @@ import pytest
 
 import demo_matrixfree_csem_gb300 as cs
 from cases import oracle_for, probe, product_grid, relerr
-from demo_matrixfree_csem_gb300 import synthetic
+from demo_matrixfree_csem_gb300 import api, synthetic
 from test_gpu_grouped_sweeps import _lusgs_batch
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +65,25 @@ def test_large_batches_give_each_system_its_own_bits(gpu, tmp_path, shape):
     got = _lusgs_batch(ctx, freqs, X)
     for q in (0, 1, 16, 31, 32):
         assert np.array_equal(got[q], _lusgs_batch(ctx, freqs[q:q + 1], X[q:q + 1])[0])
+
+
+@pytest.mark.parametrize("airbc,fvm", [(0, 0), (1, 1)])
+@pytest.mark.parametrize("shape", SHAPES[:4], ids=["x".join(map(str, s)) for s in SHAPES[:4]])
+def test_output_of_any_content_is_overwritten(gpu, tmp_path, shape, airbc, fvm):
+    """Only the boundary edges of y are cleared beforehand: the rest must not be read."""
+    import ctypes as C
+
+    import torch
+    ctx, _ = _setup(tmp_path, 96, shape, airbc, fvm)
+    x = torch.from_numpy(np.stack([probe(ctx.lE, 7 + q) for q in range(3)]).astype(np.complex64)).cuda()
+    z = cs.iom_of(0.75)
+    iom = np.array([z.real, z.imag] * 3)
+    out = []
+    for fill in (0.0, float("nan")):
+        y = torch.full_like(x, complex(fill, fill))
+        torch.cuda.synchronize()
+        assert api.lib().csem_lusgs_apply_dev(ctx.h, 32, 3, iom.ctypes.data_as(C.POINTER(C.c_double)),
+                                                 C.c_void_p(x.data_ptr()), C.c_void_p(y.data_ptr()), None) == 0
+        torch.cuda.synchronize()
+        out.append(y.cpu().numpy())
+    assert np.isfinite(out[1]).all() and np.array_equal(out[0], out[1])
