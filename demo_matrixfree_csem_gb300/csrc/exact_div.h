@@ -102,26 +102,45 @@ CSEM_HD double xd_div(double a, double d, uint64_t R, uint32_t& bad)
   return zero ? a : xd_double(res);
 }
 
-#ifdef __CUDACC__
-// The same for a divisor that is only known now, of either sign: R from the correctly
-// rounded FP64 reciprocal has 53 good bits, so q is off by at most one either way and the
-// remainder is signed.
+// The same for a divisor that is only known now, of either sign: R by Newton's iteration on
+// integers, from a single precision reciprocal (23 bits; 44 after one step, 60 after two). q is
+// off by at most one either way, and the remainder is signed. 30 integer instructions; the FP64
+// unit's own reciprocal costs it 9 operations, in a chain.
 struct XdDen {
   double d;
   uint64_t R;
 };
-__device__ __forceinline__ XdDen xd_den(double d, uint32_t& bad)
+CSEM_HD XdDen xd_den(double d, uint32_t& bad)
 {
   XdDen n;
   n.d = d;
-  const uint32_t hi = (uint32_t)__double2hiint(d);
+  const uint64_t u = xd_bits(d);
+  const uint32_t hi = (uint32_t)(u >> 32), lo = (uint32_t)u;
   bad |= xd_in_range(hi) ? 0u : 1u;
-  const uint64_t y = xd_bits(__drcp_rn(fabs(d)));
-  const bool p2 = (xd_bits(d) << 12) == 0;
-  n.R = p2 ? ~0ull : ((y & 0xfffffffffffffull) | (1ull << 52)) << 11;
+  const uint64_t D = (((uint64_t)((hi & 0xfffffu) | 0x100000u) << 32) | lo) << 11;  // 2^63 times 1 <= d' < 2
+  const uint32_t f = 0x3f800000u | (hi & 0xfffffu) << 3 | lo >> 29;
+#ifdef __CUDA_ARCH__
+  float r = __fdividef(1.f, __uint_as_float(f));
+  r = fminf(fmaxf(r, 0.5f), 0.99999994f);
+  const uint32_t x = (__float_as_uint(r) << 8) | 0x80000000u;  // 2^32 / d'
+#else
+  float g, r;
+  memcpy(&g, &f, 4);
+  r = 1.f / g;
+  r = r < 0.5f ? 0.5f : (r > 0.99999994f ? 0.99999994f : r);
+  uint32_t x;
+  memcpy(&x, &r, 4);
+  x = (x << 8) | 0x80000000u;
+#endif
+  // y ~ 2^63 / d', and 2^62 - D y / 2^64 the error times 2^62
+  uint64_t y = (uint64_t)x << 31;
+  const int64_t e = (int64_t)(1ull << 62) - (int64_t)xd_mulhi(D, y);  // below 2^41 in size
+  y += (uint64_t)(((int64_t)x * (int32_t)(e >> 10)) >> 21);
+  const int64_t e1 = (int64_t)(1ull << 62) - (int64_t)xd_mulhi(D, y);  // below 2^20
+  y += (uint64_t)(((int64_t)(uint32_t)(y >> 32) * (int32_t)e1) >> 30);
+  n.R = (u << 12) == 0 || y >> 63 ? ~0ull : y << 1;
   return n;
 }
-#endif
 CSEM_HD double xd_div2(double a, double d, uint64_t R, uint32_t& bad)
 {
   const uint64_t u = xd_bits(a), v = xd_bits(d);

@@ -5,9 +5,10 @@
 // (fdfd.c:347-503). In the coupled plane (row r, march m) a point depends on (r-1, m) and
 // (r, m-1) (forward; r+1 and m+1 backward); the third axis is independent:
 //   Ex: rows k, march j, lines i    Ey: rows k, march i, lines j    Ez: rows j, march i, lines k
-// One CTA owns one line of one system and gives every row a thread; rows advance in
-// lockstep, skewed by one step per row, and a row's value reaches the next row by a warp
-// shuffle or the hand-over between warps (k_sweep_common.cuh).
+// One CTA owns one line of one system and gives every row two threads (one above 256 rows). One
+// takes the steps: rows advance in lockstep, skewed by one step per row, and a row's value
+// reaches the next row by a warp shuffle or a hand-over between warps. The other makes, a step
+// ahead, what the step takes that no row writes during the sweep, and leaves it in shared memory.
 //
 // The reference's update (fdfd.c:358-369, 384-395, 410-421; own = 0 at the point) is, for
 // the three components alike,
@@ -27,11 +28,14 @@
 //   - products with iwmu, whose real part is zero, take 2 multiplications instead of 6
 //     operations, and p0 of a step is p1 of its neighbour step, kept in registers;
 //   - everything that no other row writes during the sweep (p0, p1, lo/dsm, Smith's ratio
-//     and denominator) is formed one step ahead, off the dependent chain.
+//     and denominator) is formed one step ahead, off the dependent chain, by other warps: 1000
+//     to 3700 cycles of a step next to the 2700 to 3500 of the chain, instead of after them.
 // A point whose operands leave exact_div.h's range (subnormal, infinite, NaN), or any point
 // where iwmu has a real part, takes the reference's operations as they stand (slow_point).
-// 120 x 120 x 120 cells, one system: 4.1 ms an application, 20.0 ms with the FP64 unit's
-// divisions (1.86 and 9.7 ms each where three systems' applications overlap).
+// 120 x 120 x 120 cells, one system: 2.95 ms an application; 3.9 ms with one thread a row and the
+// FP64 unit's reciprocal of the denominator, 20.0 ms with its divisions (1.54, 1.85 and 9.7 ms
+// each where three systems' applications overlap). 128 registers let two lines onto an SM; with
+// up to 204 one system takes 2.71 ms, but three 2.15 each.
 #include "csem_cuda.cuh"
 #include "engine.h"
 #include "exact_div.h"
@@ -100,6 +104,84 @@ __device__ __noinline__ C slow_point(const Raw& m, const Raw& r, double line_ds,
   return cdiv<F64>(csub<F64>(b, aij), aii);
 }
 
+// A row of a line (r along the row axis): pointers to its own component, the lower row, and the
+// coupled components on the upper (A) and lower (B) side of the line, for the march axis (m*)
+// and, at this row and the lower one, for the row axis (r*); and its spacings
+template <int COMP, bool PHI> struct Row {
+  C* own;
+  const C *low, *mA, *mB, *rA, *rB, *rC, *rD, *bb, *v1 = nullptr, *v0 = nullptr;  // v: node potential at the edge's two ends
+  const double* sg0;
+  Sp ln;
+  Ax64 Ra;
+  __device__ __forceinline__ Row(const SweepP<F64>& s, int slot, int sys, int line, int r)
+  {
+    const GridP<F64>& g = s.g;
+    const int n1 = g.n1, n2 = g.n2;
+    const View<F64> V = view_of<F64>(s, slot, sys);
+    const int k = COMP == 2 ? line : r, j = COMP == 0 ? 0 : (COMP == 1 ? line : r), i0 = COMP == 0 ? line : 0;
+    ln = COMP == 0 ? sp(g.d1s, g.q1s, line) : (COMP == 1 ? sp(g.d2s, g.q2s, line) : sp(g.d3s, g.q3s, line));
+    Ra = COMP == 2 ? ax64(g.d2, g.d2s, g.q2, g.q2s, r) : ax64(g.d3, g.d3s, g.q3, g.q3s, r);
+    own = V.row(COMP, k, j) + i0;
+    low = COMP == 2 ? V.row(2, k, j - 1) : V.row(COMP, k - 1, j) + i0;
+    if (COMP == 0) {
+      mB = V.row(1, k, 0) + i0, mA = mB + 1;
+      rB = V.row(2, k, 0) + i0, rA = rB + 1;
+      rD = V.row(2, k - 1, 0) + i0, rC = rD + 1;
+    } else if (COMP == 1) {
+      mA = V.row(0, k, j + 1), mB = V.row(0, k, j);
+      rA = V.row(2, k, j + 1), rB = V.row(2, k, j);
+      rC = V.row(2, k - 1, j + 1), rD = V.row(2, k - 1, j);
+    } else {
+      mA = V.row(0, k + 1, j), mB = V.row(0, k, j);
+      rA = V.row(1, k + 1, j), rB = V.row(1, k, j);
+      rC = V.row(1, k + 1, j - 1), rD = V.row(1, k, j - 1);
+    }
+    bb = V.brow(COMP, k, j);
+    if (bb) bb += i0;
+    sg0 = COMP == 0 ? g.s11 + ix1(n1, n2, k, 0, i0)
+                    : (COMP == 1 ? g.s22 + ix2(n1, n2, k, j, 0) : g.s33 + ix3(n1, n2, k, j, 0));
+    if (PHI) {
+      const C* vp = s.V + (size_t)slot * s.lv;
+      v0 = vp + ix3(n1, n2, k, j, i0);
+      v1 = COMP == 0 ? v0 + 1 : (COMP == 1 ? vp + ix3(n1, n2, k, j + 1, 0) : vp + ix3(n1, n2, k + 1, j, 0));
+    }
+  }
+  // spacings of the march axis at position m, and the cell volume (Ex's for all three
+  // components, fdfd.c:365,391,417)
+  static __device__ __forceinline__ Ax64 march(const GridP<F64>& g, int m)
+  {
+    return COMP == 0 ? ax64(g.d2, g.d2s, g.q2, g.q2s, m) : ax64(g.d1, g.d1s, g.q1, g.q1s, m);
+  }
+  __device__ __forceinline__ double volume(const GridP<F64>& g, int line, const Ax64& Ma) const
+  {
+    const double xs = COMP == 0 ? ln.d : Ma.s.d;
+    const double yd = COMP == 0 ? Ma.c.d : (COMP == 1 ? ro(g.d2 + line) : Ra.c.d);
+    return F64::mul(F64::mul(xs, yd), COMP == 2 ? ro(g.d3 + line) : Ra.c.d);
+  }
+};
+
+// the whole point (row r, march position m) again by the reference's operations
+template <int COMP, bool FWD, bool PHI>
+__device__ __noinline__ C slow_row(const SweepP<F64>& s, int slot, int sys, int line, int r, int m_, C prev, C nb)
+{
+  constexpr bool HASM = COMP != 0 || !FWD, HASR = COMP == 2 || !FWD;
+  const GridP<F64>& g = s.g;
+  const Row<COMP, PHI> W(s, slot, sys, line, r);
+  const SysScal<F64> sc = s.scal[sys];
+  const C z = make_double2(0, 0);
+  const long m = m_, so = COMP == 0 ? g.n1 : 1, sm = COMP == 0 ? g.n1 + 1 : 1;
+  Raw qm{FWD ? z : prev, FWD ? prev : W.own[(m - 1) * so], z, z, z, z};
+  Raw qr{FWD ? z : nb, FWD ? nb : W.low[m * so], z, z, z, z};
+  if (HASM) qm.A = ro(W.mA + m * sm), qm.B = ro(W.mB + m * sm), qm.Cc = ro(W.mA + (m - 1) * sm), qm.D = ro(W.mB + (m - 1) * sm);
+  if (HASR) qr.A = ro(W.rA + m * sm), qr.B = ro(W.rB + m * sm), qr.Cc = ro(W.rC + m * sm), qr.D = ro(W.rD + m * sm);
+  const double sg = ro(W.sg0 + m * so);
+  const C ee = PHI ? rmul<F64>(sg, cdivr<F64>(csub<F64>(ro(W.v1 + m * sm), ro(W.v0 + m * sm)), W.ln.d)) : z;
+  const Ax64 A = W.march(g, m_);
+  const double gg = F64::add(COMP == 0 ? ro(g.g2 + m) : ro(g.g1 + m), COMP == 2 ? ro(g.g2 + r) : ro(g.g3 + r));
+  return slow_point(qm, qr, W.ln.d, A.s.d, A.sm.d, A.c.d, W.Ra.s.d, W.Ra.sm.d, W.Ra.c.d, gg, sg, W.volume(g, line, A),
+                    g.fvm, W.bb ? ro(W.bb + m * so) : z, ee, sc.iwmu, sc.iom);
+}
+
 // Smith's quotient by aii in two parts: what depends on aii alone, and the rest
 struct Den {
   double r;     // the smaller part of aii over the larger
@@ -146,72 +228,38 @@ __global__ void k_diag64(SweepP<F64> s, ulonglong2* T)
   T[(size_t)blockIdx.y * e3 + q] = t;
 }
 
+constexpr int TRAY = 11;  // 16-byte fields of a step's operands
+
 // grid (lines, slots). APHI: A-phi's edge sweep, whose backward pass adds sigma grad v
-template <int COMP, bool FWD, bool APHI, int MAXR>
-__global__ void __launch_bounds__(MAXR, 1) k_sweep64(SweepP<F64> s, const ulonglong2* __restrict__ T)
+template <int COMP, bool FWD, bool APHI, int MAXR, bool PAIR>
+__global__ void __launch_bounds__(PAIR ? 2 * MAXR : MAXR, PAIR && MAXR <= 128 ? 2 : 1)
+    k_sweep64(const __grid_constant__ SweepP<F64> s, const ulonglong2* __restrict__ T)
 {
-  __shared__ HandOff<1, C, (MAXR <= NB_ROWS)> hand;
   const int slot = blockIdx.y;
   const int sys = s.sys_list ? s.sys_list[slot] : slot;
   const GridP<F64>& g = s.g;
   const int n1 = g.n1, n2 = g.n2, nK = s.nK;
   const int line = blockIdx.x;
-  const View<F64> V = view_of<F64>(s, slot, sys);
   const SysScal<F64> sc = s.scal[sys];
   const C z = make_double2(0, 0);
   constexpr bool HASM = COMP != 0 || !FWD;  // the coupling along the march axis is not zero
   constexpr bool HASR = COMP == 2 || !FWD;  // and along the row axis
   constexpr bool PHI = APHI && !FWD;
   const int R_ = COMP == 2 ? n2 - 1 : nK - 1, M = COMP == 0 ? n2 - 1 : n1 - 1;
-  const int rr = threadIdx.x;
+  const int rows = PAIR ? blockDim.x / 2 : blockDim.x;
+  const bool first = PAIR && threadIdx.x >= rows;  // a row's second thread, which makes the step's operands
+  const int rr = threadIdx.x - (first ? rows : 0);
   const bool rowok = rr < R_;
   const int r = rowok ? (FWD ? 1 + rr : R_ - rr) : 1;
-  const int k = COMP == 2 ? line : r, j = COMP == 0 ? 0 : (COMP == 1 ? line : r), i0 = COMP == 0 ? line : 0;
   const bool fast = g.q1 != nullptr && sc.iwmu.x == 0. && sc.iom.x == 0.;
   const double wy = sc.iwmu.y;
 
-  const Sp ln = COMP == 0 ? sp(g.d1s, g.q1s, line) : (COMP == 1 ? sp(g.d2s, g.q2s, line) : sp(g.d3s, g.q3s, line));
-  const Ax64 Ra = COMP == 2 ? ax64(g.d2, g.d2s, g.q2, g.q2s, r) : ax64(g.d3, g.d3s, g.q3, g.q3s, r);
-  // this row: own component, the lower row, and the coupled components on the upper (A)
-  // and lower (B) side of the line, for the march axis (m*) and, at this row and the lower
-  // one, for the row axis (r*); strides along the march
-  const long so = COMP == 0 ? n1 : 1, sm = COMP == 0 ? n1 + 1 : 1;
-  C* own = V.row(COMP, k, j) + i0;
-  const C* low = COMP == 2 ? V.row(2, k, j - 1) : V.row(COMP, k - 1, j) + i0;
-  const C *mA, *mB, *rA, *rB, *rC, *rD;
-  if (COMP == 0) {
-    mB = V.row(1, k, 0) + i0, mA = mB + 1;
-    rB = V.row(2, k, 0) + i0, rA = rB + 1;
-    rD = V.row(2, k - 1, 0) + i0, rC = rD + 1;
-  } else if (COMP == 1) {
-    mA = V.row(0, k, j + 1), mB = V.row(0, k, j);
-    rA = V.row(2, k, j + 1), rB = V.row(2, k, j);
-    rC = V.row(2, k - 1, j + 1), rD = V.row(2, k - 1, j);
-  } else {
-    mA = V.row(0, k + 1, j), mB = V.row(0, k, j);
-    rA = V.row(1, k + 1, j), rB = V.row(1, k, j);
-    rC = V.row(1, k + 1, j - 1), rD = V.row(1, k, j - 1);
-  }
-  const C* bb = V.brow(COMP, k, j);
-  if (bb) bb += i0;
-  const double* sg0 = COMP == 0 ? g.s11 + ix1(n1, n2, k, 0, i0)
-                                : (COMP == 1 ? g.s22 + ix2(n1, n2, k, j, 0) : g.s33 + ix3(n1, n2, k, j, 0));
+  const Row<COMP, PHI> W(s, slot, sys, line, r);
+  const long so = COMP == 0 ? n1 : 1, sm = COMP == 0 ? n1 + 1 : 1;  // strides along the march
   const ulonglong2* tab = T + (size_t)slot * diag64_entries(n1, n2, nK);
   if (COMP == 0) tab += (long)r * (n2 + 1);
   else tab += (long)(nK + 1) * (n2 + 1) + (COMP == 2 ? (long)(nK + 1) * (n1 + 1) : 0) + (long)r * (n1 + 1);
-  const C *v1 = nullptr, *v0 = nullptr;  // node potential at the edge's two ends
-  if (PHI) {
-    const C* vp = s.V + (size_t)slot * s.lv;
-    v0 = vp + ix3(n1, n2, k, j, i0);
-    v1 = COMP == 0 ? v0 + 1 : (COMP == 1 ? vp + ix3(n1, n2, k, j + 1, 0) : vp + ix3(n1, n2, k + 1, j, 0));
-  }
   auto at = [&](int c) { return FWD ? 1 + c : M - c; };
-  // (cell volume: Ex's for all three components, fdfd.c:365,391,417)
-  auto volume = [&](const Ax64& Ma) {
-    const double xs = COMP == 0 ? ln.d : Ma.s.d;
-    const double yd = COMP == 0 ? Ma.c.d : (COMP == 1 ? ro(g.d2 + line) : Ra.c.d);
-    return F64::mul(F64::mul(xs, yd), COMP == 2 ? ro(g.d3 + line) : Ra.c.d);
-  };
 
   // operands of the next step
   C lb = z, pA = z, pB = z, qA = z, qB = z, qC = z, qD = z, lom = z, lor = z, va = z, vb = z;
@@ -220,29 +268,29 @@ __global__ void __launch_bounds__(MAXR, 1) k_sweep64(SweepP<F64> s, const ulongl
   Ax64 Mn{};
   auto load = [&](int c) {  // nothing read here is written before that step
     const long m = at(c);
-    lb = bb ? ro(bb + m * so) : z;
-    lsg = ro(sg0 + m * so);
+    lb = W.bb ? ro(W.bb + m * so) : z;
+    lsg = ro(W.sg0 + m * so);
     lt = __ldg(tab + m);
-    Mn = COMP == 0 ? ax64(g.d2, g.d2s, g.q2, g.q2s, (int)m) : ax64(g.d1, g.d1s, g.q1, g.q1s, (int)m);
+    Mn = W.march(g, (int)m);
     if (HASM) {  // the side that the step before did not have: upper forward, lower backward
       const long o = (FWD ? m : m - 1) * sm;
-      pA = ro(mA + o);
-      pB = ro(mB + o);
+      pA = ro(W.mA + o);
+      pB = ro(W.mB + o);
     }
     if (HASR) {
       const long o = m * sm;
-      qA = ro(rA + o);
-      qB = ro(rB + o);
-      qC = ro(rC + o);
-      qD = ro(rD + o);
+      qA = ro(W.rA + o);
+      qB = ro(W.rB + o);
+      qC = ro(W.rC + o);
+      qD = ro(W.rD + o);
     }
     if (!FWD) {  // the component's own not-yet-swept neighbours
-      lom = own[(m - 1) * so];
-      lor = low[m * so];
+      lom = W.own[(m - 1) * so];
+      lor = W.low[m * so];
     }
     if (PHI) {
-      va = ro(v1 + m * sm);
-      vb = ro(v0 + m * sm);
+      va = ro(W.v1 + m * sm);
+      vb = ro(W.v0 + m * sm);
     }
   };
   // what the step takes from them: u = p0 (minus nothing yet), w = p1 + lo/dsm per axis
@@ -257,11 +305,11 @@ __global__ void __launch_bounds__(MAXR, 1) k_sweep64(SweepP<F64> s, const ulongl
     Ma = Mn;
     if (HASM) {
       uint32_t bn = 0;
-      const C p = over(csub<F64>(pA, pB), ln, bn);
+      const C p = over(csub<F64>(pA, pB), W.ln, bn);
       if (c == 0) {
         const long o = (FWD ? (long)at(c) - 1 : (long)at(c)) * sm;
         badk = 0;
-        pk = over(csub<F64>(ro(mA + o), ro(mB + o)), ln, badk);
+        pk = over(csub<F64>(ro(W.mA + o), ro(W.mB + o)), W.ln, badk);
       }
       um = FWD ? p : pk;
       wm = FWD ? pk : p;
@@ -270,83 +318,154 @@ __global__ void __launch_bounds__(MAXR, 1) k_sweep64(SweepP<F64> s, const ulongl
       badk = bn;
     }
     if (HASR) {
-      ur = over(csub<F64>(qA, qB), ln, badp);
-      wr = over(csub<F64>(qC, qD), ln, badp);
+      ur = over(csub<F64>(qA, qB), W.ln, badp);
+      wr = over(csub<F64>(qC, qD), W.ln, badp);
     }
     if (!FWD) {
       wm = cadd<F64>(wm, over(lom, Ma.sm, badp));
-      wr = cadd<F64>(wr, over(lor, Ra.sm, badp));
+      wr = cadd<F64>(wr, over(lor, W.Ra.sm, badp));
     }
-    if (PHI) e = rmul<F64>(lsg, over(csub<F64>(va, vb), ln, badp));
+    if (PHI) e = rmul<F64>(lsg, over(csub<F64>(va, vb), W.ln, badp));
     const double ay = xd_double(lt.x);
     double x = -lsg, y = ay;
     if (g.fvm) {
-      fy = F64::mul(volume(Ma), sc.iom.y);
+      fy = F64::mul(W.volume(g, line, Ma), sc.iom.y);
       x = -F64::mul(ay, fy);
       y = -F64::mul(lsg, fy);
     } else {
       badp |= lt.y == 0 ? 1u : 0u;
     }
-    den.ydom = fabs(x) < fabs(y);
-    if (den.ydom && !g.fvm) den.r = xd_div2(x, ay, lt.y, badp);
-    else den.r = den.ydom ? F64::div(x, y) : F64::div(y, x);
+    den.ydom = xd_bits(x) << 1 < xd_bits(y) << 1;  // |x| < |y|
+    if (den.ydom && !g.fvm) {
+      den.r = xd_div2(x, ay, lt.y, badp);
+    } else {
+      const XdDen n = xd_den(den.ydom ? y : x, badp);
+      den.r = xd_div2(den.ydom ? x : y, n.d, n.R, badp);
+    }
     den.q = xd_den(F64::add(F64::mul(den.ydom ? x : y, den.r), den.ydom ? y : x), badp);
   };
-  // the whole point again by the reference's operations
-  auto slow = [&](int c, C prev, C nb) {
-    const long m = at(c);
-    Raw qm{FWD ? z : prev, FWD ? prev : own[(m - 1) * so], z, z, z, z};
-    Raw qr{FWD ? z : nb, FWD ? nb : low[m * so], z, z, z, z};
-    if (HASM) qm.A = ro(mA + m * sm), qm.B = ro(mB + m * sm), qm.Cc = ro(mA + (m - 1) * sm), qm.D = ro(mB + (m - 1) * sm);
-    if (HASR) qr.A = ro(rA + m * sm), qr.B = ro(rB + m * sm), qr.Cc = ro(rC + m * sm), qr.D = ro(rD + m * sm);
-    const double sg = ro(sg0 + m * so);
-    const C ee = PHI ? rmul<F64>(sg, cdivr<F64>(csub<F64>(ro(v1 + m * sm), ro(v0 + m * sm)), ln.d)) : z;
-    const Ax64 A = COMP == 0 ? ax64(g.d2, g.d2s, g.q2, g.q2s, (int)m) : ax64(g.d1, g.d1s, g.q1, g.q1s, (int)m);
-    const double gg = F64::add(COMP == 0 ? ro(g.g2 + m) : ro(g.g1 + m), COMP == 2 ? ro(g.g2 + r) : ro(g.g3 + r));
-    return slow_point(qm, qr, ln.d, A.s.d, A.sm.d, A.c.d, Ra.s.d, Ra.sm.d, Ra.c.d, gg, sg, volume(A), g.fvm,
-                      bb ? ro(bb + m * so) : z, ee, sc.iwmu, sc.iom);
-  };
-
-  C res[1] = {z};
-  if (fast && rowok && rr == 0 && M > 0) {
-    load(0);
-    make(0);
-  }
-  for (int t = 0; t < M + R_ - 1; t++) {
-    const int c = t - rr;
-    const bool act = rowok && c >= 0 && c < M;
-    const bool nxt = fast && rowok && c + 1 >= 0 && c + 1 < M;
-    if (nxt) load(c + 1);
-    const C prev = c > 0 ? res[0] : z;  // own row, previous march position
+  // one step of a row: prev is its value at the march position before, nb the row before's at
+  // this one
+  auto step = [&](int c, C prev, C nb) {
     uint32_t bad = fast ? badp : 1u;
-    C Lm = z;
-    if (act && fast) {  // the march axis before the previous row's value arrives
-      const C em = over(prev, FWD ? Ma.sm : Ma.s, bad);
-      Lm = over(FWD ? csub<F64>(um, cadd<F64>(wm, em)) : csub<F64>(csub<F64>(um, em), wm), Ma.c, bad);
+    C v = z;
+    if (fast) {  // (both axes at a time: their chains are as long)
+      const C em = over(prev, FWD ? Ma.sm : Ma.s, bad), er = over(nb, FWD ? W.Ra.sm : W.Ra.s, bad);
+      const C Lm = over(FWD ? csub<F64>(um, cadd<F64>(wm, em)) : csub<F64>(csub<F64>(um, em), wm), Ma.c, bad);
+      const C Lr = over(FWD ? csub<F64>(ur, cadd<F64>(wr, er)) : csub<F64>(csub<F64>(ur, er), wr), W.Ra.c, bad);
+      const C S = cadd<F64>(Lm, Lr);
+      C a = make_double2(-F64::mul(S.y, wy), F64::mul(S.x, wy));
+      if (PHI) a = csub<F64>(a, e);
+      if (g.fvm) a = make_double2(-F64::mul(a.y, fy), F64::mul(a.x, fy));
+      v = smith(csub<F64>(b, a), den, bad);
     }
-    C nb[1];
-    hand.get(res, nb, t);
-    if (act) {
-      C v = z;
-      if (fast) {
-        const C er = over(nb[0], FWD ? Ra.sm : Ra.s, bad);
-        const C Lr = over(FWD ? csub<F64>(ur, cadd<F64>(wr, er)) : csub<F64>(csub<F64>(ur, er), wr), Ra.c, bad);
-        const C S = cadd<F64>(Lm, Lr);
-        C a = make_double2(-F64::mul(S.y, wy), F64::mul(S.x, wy));
-        if (PHI) a = csub<F64>(a, e);
-        if (g.fvm) a = make_double2(-F64::mul(a.y, fy), F64::mul(a.x, fy));
-        v = smith(csub<F64>(b, a), den, bad);
+    if (bad) v = slow_row<COMP, FWD, PHI>(s, slot, sys, line, r, at(c), prev, nb);
+    W.own[(long)at(c) * so] = v;
+    return v;
+  };
+  const int steps = M + R_ - 1;
+  if constexpr (PAIR) {
+    extern __shared__ ulonglong2 smem[];
+    // a step's operands, [parity][field][row], and the last rows of the warps, [parity][warp]
+    ulonglong2* const tray = smem + rr;
+    C* const last = (C*)(smem + 2 * TRAY * rows);
+    const int lane = threadIdx.x & 31, w = rr >> 5, nw = rows >> 5;
+    // up to 4 warps hand over by named barriers (1 .. 6) and meet their second warps at 7 .. 10
+    constexpr bool NAMED = MAXR <= 128;
+    auto meet = [&]() {
+      if constexpr (NAMED) nbar_sync(7 + w);
+      else __syncthreads();
+    };
+    auto put = [&](ulonglong2*& p, double x, double y) {
+      *p = make_ulonglong2(xd_bits(x), xd_bits(y));
+      p += rows;
+    };
+    auto take = [&](const ulonglong2*& p) {
+      const ulonglong2 u = *p;
+      p += rows;
+      return make_double2(xd_double(u.x), xd_double(u.y));
+    };
+    if (first) {
+      if (fast && rowok && rr == 0 && M > 0) load(0);
+      for (int t = -1; t < steps; t++) {
+        const int c = t + 1 - rr;
+        if (fast && rowok && c >= 0 && c < M) {
+          make(c);
+          ulonglong2* p = tray + (t + 1 & 1) * TRAY * rows;
+          put(p, b.x, b.y);
+          if (HASM || !FWD) put(p, um.x, um.y), put(p, wm.x, wm.y);
+          if (HASR || !FWD) put(p, ur.x, ur.y), put(p, wr.x, wr.y);
+          if (PHI) put(p, e.x, e.y);
+          const Sp msp = FWD ? Ma.sm : Ma.s;
+          put(p, msp.d, xd_double(msp.R));
+          put(p, Ma.c.d, xd_double(Ma.c.R));
+          put(p, den.r, den.q.d);
+          put(p, xd_double(den.q.R), xd_double((badp ? 1u : 0u) | (den.ydom ? 2u : 0u)));
+          if (g.fvm) put(p, fy, 0.);
+        }
+        if (fast && rowok && c + 1 >= 0 && c + 1 < M) load(c + 1);
+        meet();
       }
-      if (bad) v = slow(c, prev, nb[0]);
-      own[(long)at(c) * so] = v;
-      res[0] = v;
-    } else {
-      res[0] = z;
+      return;
     }
-    hand.put(res, t);
-    if (nxt) make(c + 1);
+    C res = z;
+    meet();
+    for (int t = 0; t < steps; t++) {
+      const int c = t - rr;
+      C nb = make_double2(__shfl_up_sync(0xffffffffu, res.x, 1), __shfl_up_sync(0xffffffffu, res.y, 1));
+      const bool wait = NAMED && w > 0 && t > 0;
+      if (wait) nbar_sync(2 * w - 1);  // the warp before has written step t - 1
+      if (lane == 0) nb = w > 0 && t > 0 ? last[(NAMED ? 0 : (t - 1 & 1) * nw) + w - 1] : z;
+      if (wait) nbar_arrive(2 * w);  // and may write step t
+      if (rowok && c >= 0 && c < M) {
+        if (fast) {
+          const ulonglong2* p = tray + (t & 1) * TRAY * rows;
+          b = take(p);
+          if (HASM || !FWD) um = take(p), wm = take(p);
+          if (HASR || !FWD) ur = take(p), wr = take(p);
+          if (PHI) e = take(p);
+          C q = take(p);
+          (FWD ? Ma.sm : Ma.s).d = q.x, (FWD ? Ma.sm : Ma.s).R = xd_bits(q.y);
+          q = take(p);
+          Ma.c.d = q.x, Ma.c.R = xd_bits(q.y);
+          q = take(p);
+          den.r = q.x, den.q.d = q.y;
+          q = take(p);
+          den.q.R = xd_bits(q.x);
+          badp = (uint32_t)xd_bits(q.y) & 1, den.ydom = (xd_bits(q.y) & 2) != 0;
+          if (g.fvm) fy = take(p).x;
+        }
+        res = step(c, c > 0 ? res : z, nb);
+      } else {
+        res = z;
+      }
+      const bool next = NAMED && w + 1 < nw;
+      if (next && t > 0) nbar_sync(2 * w + 2);  // the next warp has read step t - 1
+      if (lane == 31) last[(NAMED ? 0 : (t & 1) * nw) + w] = res;
+      if (next) nbar_arrive(2 * w + 1);
+      meet();
+    }
+    if (NAMED && w > 0 && steps > 0) nbar_sync(2 * w - 1);  // the barriers' last generation
+  } else {
+    __shared__ HandOff<1, C, (MAXR <= NB_ROWS)> hand;
+    C res[1] = {z};
+    if (fast && rowok && rr == 0 && M > 0) {
+      load(0);
+      make(0);
+    }
+    for (int t = 0; t < steps; t++) {
+      const int c = t - rr;
+      const bool act = rowok && c >= 0 && c < M;
+      const bool nxt = fast && rowok && c + 1 >= 0 && c + 1 < M;
+      if (nxt) load(c + 1);
+      C nb[1];
+      hand.get(res, nb, t);
+      res[0] = act ? step(c, c > 0 ? res[0] : z, nb[0]) : z;
+      hand.put(res, t);
+      if (nxt) make(c + 1);
+    }
+    hand.finish(steps);
   }
-  hand.finish(M + R_ - 1);
 }
 
 template <int COMP, bool FWD, bool APHI>
@@ -355,8 +474,18 @@ static void launch64(const SweepP<F64>& s, int nslot, const ulonglong2* T, cudaS
   const int rows = COMP == 2 ? s.g.n2 - 1 : s.nK - 1;
   const int threads = (rows + 31) / 32 * 32;
   dim3 grd(COMP == 0 ? s.g.n1 : (COMP == 1 ? s.g.n2 : s.nK), nslot);
-  if (rows > NB_ROWS) count_launch(), k_sweep64<COMP, FWD, APHI, MAXROWS><<<grd, threads, 0, st>>>(s, T);
-  else count_launch(), k_sweep64<COMP, FWD, APHI, NB_ROWS><<<grd, threads, 0, st>>>(s, T);
+  // two threads a row while a CTA can hold them
+  const size_t sm = (size_t)threads * 2 * TRAY * 16 + 2 * (threads / 32) * 16;
+  count_launch();
+  if (rows > NB_ROWS) {
+    k_sweep64<COMP, FWD, APHI, MAXROWS, false><<<grd, threads, 0, st>>>(s, T);
+  } else if (rows > 128) {
+    allow_smem<k_sweep64<COMP, FWD, APHI, NB_ROWS, true>>(sm);
+    k_sweep64<COMP, FWD, APHI, NB_ROWS, true><<<grd, 2 * threads, sm, st>>>(s, T);
+  } else {
+    allow_smem<k_sweep64<COMP, FWD, APHI, 128, true>>(sm);
+    k_sweep64<COMP, FWD, APHI, 128, true><<<grd, 2 * threads, sm, st>>>(s, T);
+  }
 }
 
 size_t sweep64_table_bytes(int n1, int n2, int nK) { return sizeof(ulonglong2) * (size_t)diag64_entries(n1, n2, nK); }
