@@ -96,6 +96,8 @@ void launch_sweep_pipelined(const SweepP<F32>& s, int comp, bool fwd, int nslot,
 void launch_sweep64(const SweepP<F64>& s, int comp, bool fwd, bool aphi, int nslot, const void* T, cudaStream_t st);
 void launch_sweep64_table(const SweepP<F64>& s, int nslot, void* T, cudaStream_t st);
 size_t sweep64_table_bytes(int n1, int n2, int nK);
+// launch_aphi_phi<F64> with the quotients on the integer units (spacings in range, not aphi_fix)
+void launch_aphi_phi64(const SweepP<F64>& s, double2* V, int t, int nslot, cudaStream_t st);
 bool sweep_pipelined_fits(int comp, int n1, int n2, int nK);  // the sweep's rows fit one CTA
 // complex64 line-tiled sweeps (k_lusgs3.cu): 32 lines per CTA, rows in warp blocks of at
 // most rows_per_warp (4, 8, 16), vw march positions per step for Ey/Ez (1, 2, 4)

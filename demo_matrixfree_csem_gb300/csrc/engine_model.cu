@@ -640,8 +640,14 @@ void Ops<P>::apply_aphi(const C* X, C* Y, int nslot, const int* sys_list, const 
   };
   for (int comp = 0; comp < 3; comp++) edges(comp, true);
   const int np = phi_diagonals(n1, n2, n3);
-  for (int t = 3; t < 3 + np; t++) launch_aphi_phi<P>(s, V.as<C>(), t, nslot, st);
-  for (int t = 2 + np; t >= 3; t--) launch_aphi_phi<P>(s, V.as<C>(), -t, nslot, st);
+  auto nodes = [&](int t) {
+    if constexpr (P::exact) {
+      if (pipelined_sweeps && s.g.q1 && !aphi_fix) return launch_aphi_phi64(s, V.as<C>(), t, nslot, st);
+    }
+    launch_aphi_phi<P>(s, V.as<C>(), t, nslot, st);
+  };
+  for (int t = 3; t < 3 + np; t++) nodes(t);
+  for (int t = 2 + np; t >= 3; t--) nodes(-t);
   for (int comp = 2; comp >= 0; comp--) edges(comp, false);
   launch_aphi_grad<P>(s, V.as<C>(), nslot, st);
 }

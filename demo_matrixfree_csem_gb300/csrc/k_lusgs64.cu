@@ -468,6 +468,73 @@ __global__ void __launch_bounds__(PAIR ? 2 * MAXR : MAXR, PAIR && MAXR <= 128 ? 
   }
 }
 
+// One hyperplane i + j + k = t of A-phi's node sweep (fdfd.c:654-710), as k_aphi_phi with
+// quotients on the integer units: of its 29 divisions per node the node's own diagonal is a sum of
+// host-made terms, and the others take no FP64 operation. A node where a quotient is out of range
+// is done again with the / operator. What is left is bound by latency, at some 6 us a hyperplane
+// (84^3 cells: 17 with the divisions; 474 hyperplanes an application, which takes 5.2 ms instead
+// of 10.7, 2.4 instead of 4.4 where three overlap).
+template <bool FWD>
+__global__ void __launch_bounds__(128) k_aphi_phi64(const __grid_constant__ SweepP<F64> s, C* __restrict__ VV, int t)
+{
+  const int slot = blockIdx.z;
+  const GridP<F64>& g = s.g;
+  const int n1 = g.n1, n2 = g.n2, n3 = g.n3;
+  const int i = 1 + blockIdx.x * 32 + threadIdx.x, j = 1 + blockIdx.y * 4 + threadIdx.y, k = t - i - j;
+  if (i >= n1 || j >= n2 || k < 1 || k >= n3) return;
+  const int sys = s.sys_list ? s.sys_list[slot] : slot;
+  C* v = VV + (size_t)slot * s.lv;
+  const long q = ix3(n1, n2, k, j, i), qj = ix3(n1, n2, k, j - 1, i), qk = ix3(n1, n2, k - 1, j, i);
+  const C* ax = s.Y + (size_t)sys * g.lE;
+  const C *ay = ax + g.lEx, *az = ay + g.lEy;
+  const C z = make_double2(0, 0);
+  const Ax64 X = ax64(g.d1, g.d1s, g.q1, g.q1s, i), Y = ax64(g.d2, g.d2s, g.q2, g.q2s, j), Z = ax64(g.d3, g.d3s, g.q3, g.q3s, k);
+  const double geo = F64::add(F64::add(ro(g.g1 + i), ro(g.g2 + j)), ro(g.g3 + k));
+  const C b = ro(s.BV + (size_t)slot * s.lv + q);
+  const SysScal<F64> sc = s.scal[sys];
+  auto node = [&](auto over_) {
+    // sigma (a + (hi - lo) / ds) on a face; v is zero at the node itself
+    auto face = [&](double sg, C a, C dv, Sp ds) { return rmul<F64>(sg, cadd<F64>(a, over_(dv, ds))); };
+    auto axis = [&](C up, C lo, double sp, double sm, C ap, C am, const Ax64& A) {
+      return over_(csub<F64>(face(sp, ap, up, A.s), face(sm, am, csub<F64>(z, lo), A.sm)), A.c);
+    };
+    const C x = axis(FWD ? z : v[ix3(n1, n2, k, j, i + 1)], v[q - 1], ro(g.s11 + ix1(n1, n2, k, j, i)),
+                     ro(s.s11u + ix1(n1, n2, k, j, i - 1)), ro(ax + ix1(n1, n2, k, j, i)), ro(ax + ix1(n1, n2, k, j, i - 1)), X);
+    const C y = axis(FWD ? z : v[ix3(n1, n2, k, j + 1, i)], v[qj], ro(g.s22 + ix2(n1, n2, k, j, i)),
+                     ro(s.s22u + ix2(n1, n2, k, j - 1, i)), ro(ay + ix2(n1, n2, k, j, i)), ro(ay + ix2(n1, n2, k, j - 1, i)), Y);
+    const C w = axis(FWD ? z : v[ix3(n1, n2, k + 1, j, i)], v[qk], ro(g.s33 + ix3(n1, n2, k, j, i)),
+                     ro(s.s33u + ix3(n1, n2, k - 1, j, i)), ro(az + ix3(n1, n2, k, j, i)), ro(az + ix3(n1, n2, k - 1, j, i)), Z);
+    return cadd<F64>(cadd<F64>(x, y), w);
+  };
+  uint32_t bad = 0;
+  C aij = node([&](C a, Sp d) { return over(a, d, bad); });
+  C r = z;
+  if (!g.fvm) {
+    const XdDen n = xd_den(-geo, bad);
+    const C a = csub<F64>(b, aij);
+    r = make_double2(xd_div2(a.x, n.d, n.R, bad), xd_div2(a.y, n.d, n.R, bad));
+  }
+  if (bad || g.fvm) {
+    if (bad) aij = node([&](C a, Sp d) { return cdivr<F64>(a, d.d); });
+    C aii = make_double2(-geo, 0);
+    if (g.fvm) {
+      const C f = rmul<F64>(F64::mul(F64::mul(X.s.d, Y.c.d), Z.c.d), sc.iom);
+      aij = cmul<F64>(aij, f);
+      aii = cmul<F64>(aii, f);
+    }
+    r = cdiv<F64>(csub<F64>(b, aij), aii);
+  }
+  v[q] = r;
+}
+
+void launch_aphi_phi64(const SweepP<F64>& s, double2* V, int t, int nslot, cudaStream_t st)
+{
+  const dim3 blk(32, 4), grd((s.g.n1 - 1 + 31) / 32, (s.g.n2 - 1 + 3) / 4, nslot);
+  count_launch();
+  if (t > 0) k_aphi_phi64<true><<<grd, blk, 0, st>>>(s, V, t);
+  else k_aphi_phi64<false><<<grd, blk, 0, st>>>(s, V, -t);
+}
+
 template <int COMP, bool FWD, bool APHI>
 static void launch64(const SweepP<F64>& s, int nslot, const ulonglong2* T, cudaStream_t st)
 {
