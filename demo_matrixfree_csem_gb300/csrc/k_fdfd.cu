@@ -255,7 +255,11 @@ FdfdShape fdfd_shape(int n1, int n2, int n3, int nsys, int by, int ctas_per_sm, 
   const long base = (long)f.gx * f.gy * nsys;
   // split the planes into chunks until about ctas_per_sm CTAs per SM are in the grid
   int nkc = (int)(((long)ctas_per_sm * sm_count() + base - 1) / base);
-  const int maxc = (n3 + 1) / 8 > 0 ? (n3 + 1) / 8 : 1;  // chunks of at least 8 planes
+  // chunks of at least 8 planes, as each forms H of one more; of any size where 8 leave SMs idle,
+  // and a plane's latency counts (complex128 4 us: 10^3 cells 74 us with 8 planes, 49 with 4, 35
+  // with 2, 23 with 1; 44^3 cells 74, 50, 53, 50; complex64 20 and 18)
+  const int least = base * ((n3 + 1) / 8) < sm_count() ? 1 : 8;
+  const int maxc = (n3 + 1) / least > 0 ? (n3 + 1) / least : 1;
   if (nkc > maxc) nkc = maxc;
   if (nkc < 1) nkc = 1;
   f.kchunk = (n3 + 1 + nkc - 1) / nkc;
