@@ -454,12 +454,16 @@ __global__ void __launch_bounds__(64 * LINES) k_line32(SweepP<F32> s, const floa
     }
 #pragma unroll
     for (int u = 0; u < CH; u++) {
-      const C left = make_float2(__shfl_up_sync(0xffffffffu, v.x, 1), __shfl_up_sync(0xffffffffu, v.y, 1));
+      C left = make_float2(__shfl_up_sync(0xffffffffu, v.x, 1), __shfl_up_sync(0xffffffffu, v.y, 1));
       if constexpr (starting.value) {
         const bool now = cf + u == lane;
         gp = now ? gpn : gp;
         v.x = now ? 0.f : v.x;
         v.y = now ? 0.f : v.y;
+        // lane 0 gets its own value, which gs clears, unless it comes from rows past the last,
+        // whose entries hold anything
+        left.x = lane == 0 ? 0.f : left.x;
+        left.y = lane == 0 ? 0.f : left.y;
       }
       const float gs = lane == 0 ? 0.f : gp;
       const C d = make_float2(gp * le[u].x + gn[u] * v.x, gp * le[u].y + gn[u] * v.y);

@@ -87,3 +87,16 @@ def test_output_of_any_content_is_overwritten(gpu, tmp_path, shape, airbc, fvm):
         torch.cuda.synchronize()
         out.append(y.cpu().numpy())
     assert np.isfinite(out[1]).all() and np.array_equal(out[0], out[1])
+
+
+# rows that are no multiple of 8, march positions in one strip and in several
+@pytest.mark.parametrize("shape", [(40, 37, 45, 2), (61, 5, 38, 2), (5, 62, 41, 2), (30, 29, 66, 2)], ids=lambda s: "x".join(map(str, s)))
+def test_result_does_not_depend_on_what_the_scratch_holds(gpu, tmp_path, shape):
+    """The stream's entries past the last row and position are never written, so they hold another
+    component's or another call's values; none may reach a result."""
+    freqs = [0.75, 0.5]
+    ctx, _ = _setup(tmp_path, 97, shape, 1, 0)
+    X = np.stack([probe(ctx.lE, 9 + q) for q in range(2)])
+    want = _lusgs_batch(ctx, freqs, X)
+    _lusgs_batch(ctx, freqs, np.full_like(X, complex(np.nan, np.inf)))
+    assert np.isfinite(want).all() and np.array_equal(_lusgs_batch(ctx, freqs, X), want)
