@@ -69,6 +69,17 @@ template <> struct DotAcc<F32> {
   __device__ __forceinline__ double2 value() const { return make_double2(re.value(), im.value()); }
 };
 
+// <a, a> in complex128: the real part in DotAcc<F64>'s operations and order (4 instead of 8, which
+// bind it: the imaginary part is a sum of exact zeros)
+struct NormAcc64 {
+  double acc = 0;
+  __device__ __forceinline__ void add(double2 a, double2)
+  {
+    acc = __dadd_rn(acc, __dadd_rn(__dmul_rn(a.x, a.x), __dmul_rn(a.y, a.y)));
+  }
+  __device__ __forceinline__ double2 value() const { return make_double2(acc, isfinite(acc) ? 0. : acc - acc); }
+};
+
 template <> struct DotAcc<F64Q> : DotAcc<F64> {};  // the complex128 accumulation
 
 }  // namespace
