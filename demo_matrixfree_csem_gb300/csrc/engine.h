@@ -152,6 +152,9 @@ template <class P>
 void launch_aphi_grad(const SweepP<P>& s, const typename P::C* V, int nslot, cudaStream_t st);
 
 // ---------------------------------------------------------------- BLAS-1
+// r = b - w (w null: r as it is) and out[slot] = |r|^2, complex128 by multiply-adds
+void launch_res_norm(long n, int nslot, const int* sys_list, const double2* b, const double2* w, double2* r,
+                     double2* partial, int nblk, double2* out, cudaStream_t st);
 template <class P>
 void launch_dot(const typename P::C* a, const typename P::C* b, long n, long stride, int nslot,
                 const int* sys_list, double2* partial, int nblk, double2* out, cudaStream_t st);

@@ -22,22 +22,27 @@
 
 namespace csem {
 
+constexpr int START_PER_THREAD = 4;
+
 // (r and r0 may be the same vector: the GMRES start writes r0 through both)
 __global__ void k_start_inner(long n, const int* __restrict__ list, const double* __restrict__ rn,
                               const double2* __restrict__ r64, float2* r, float2* r0, float2* __restrict__ p,
                               float2* __restrict__ d)
 {
   const int sys = list[blockIdx.y];
-  const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const size_t o = (size_t)sys * n + q;
-  const double s = 1.0 / rn[sys];
-  const double2 v = r64[o];
-  const float2 f = make_float2((float)(v.x * s), (float)(v.y * s));
-  r[o] = f;
-  r0[o] = f;
-  p[o] = f;
-  d[o] = make_float2(0.f, 0.f);
+  const size_t o = (size_t)sys * n;
+  const double s = 1.0 / rn[sys];  // (for 4 elements: the FP64 unit takes longer over it than over an element)
+#pragma unroll
+  for (int u = 0; u < START_PER_THREAD; u++) {
+    const long q = ((long)blockIdx.x * START_PER_THREAD + u) * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const double2 v = r64[o + q];
+    const float2 f = make_float2((float)(v.x * s), (float)(v.y * s));
+    r[o + q] = f;
+    r0[o + q] = f;
+    p[o + q] = f;
+    d[o + q] = make_float2(0.f, 0.f);
+  }
 }
 
 __global__ void k_outer_accum(long n, const int* __restrict__ list, const double* __restrict__ rn,
@@ -239,7 +244,7 @@ void MixedBatch::start_inner(const std::vector<int>& g, const std::vector<double
   CSEM_CUDA_TRY(cudaMemcpyAsync(list.p, g.data(), sizeof(int) * g.size(), cudaMemcpyHostToDevice, st));
   const int ng = (int)g.size();
   const int* dl = list.as<int>();
-  dim3 grd((unsigned)((n + 255) / 256), ng);
+  dim3 grd((unsigned)((n + 256 * START_PER_THREAD - 1) / (256 * START_PER_THREAD)), ng);
   count_launch(), k_start_inner<<<grd, 256, 0, st>>>(n, dl, rn.as<double>(), r64.as<double2>(), V(0), V(1), V(2), V(7));
   double2* D = dots.as<double2>();
   launch_dot2<F32>(V(0), V(1), V(0), V(0), n, n, ng, dl, partial.as<double2>(), nblk, D + 5 * nsys, D + 6 * nsys,
@@ -257,11 +262,10 @@ void MixedBatch::outer_update(const std::vector<int>& g, std::vector<double>& rn
   if (!first) {
     count_launch(), k_outer_accum<<<grd, 256, 0, st>>>(n, dl, rn.as<double>(), x64.as<double2>(), d ? d : V(7));
     o64.apply_A(x64.as<double2>(), w64.as<double2>(), ng, dl, sc64.as<SysScal<F64>>());
-    launch_vec<F64>(VEC_SUB, n, ng, dl, nullptr, b64.as<double2>(), w64.as<double2>(), r64.as<double2>(), nullptr,
-                    nullptr, st);
   }
   double2* D = dots.as<double2>();
-  launch_dot<F64>(r64.as<double2>(), r64.as<double2>(), n, n, ng, dl, partial.as<double2>(), nblk, D + 7 * nsys, st);
+  launch_res_norm(n, ng, dl, b64.as<double2>(), first ? nullptr : w64.as<double2>(), r64.as<double2>(),
+                  partial.as<double2>(), nblk, D + 7 * nsys, st);
   std::vector<double2> h(ng);
   CSEM_CUDA_TRY(cudaMemcpyAsync(h.data(), D + 7 * nsys, sizeof(double2) * ng, cudaMemcpyDeviceToHost, st));
   CSEM_CUDA_TRY(cudaStreamSynchronize(st));
@@ -639,7 +643,7 @@ void MixedBatch::gmres_inner(const std::vector<int>& g, const std::vector<double
   // r0 = r64 / |r64|, d = 0 (k_start_inner writes r, r0, p, d: here r0 twice and d)
   {
     CSEM_CUDA_TRY(cudaMemcpyAsync(list.p, g.data(), sizeof(int) * g.size(), cudaMemcpyHostToDevice, this->st));
-    dim3 grd((unsigned)((n + 255) / 256), (unsigned)g.size());
+    dim3 grd((unsigned)((n + 256 * START_PER_THREAD - 1) / (256 * START_PER_THREAD)), (unsigned)g.size());
     count_launch(), k_start_inner<<<grd, 256, 0, this->st>>>(n, list.as<int>(), rn.as<double>(), r64.as<double2>(),
                                                              GR0, GR0, GW, GD);
   }
