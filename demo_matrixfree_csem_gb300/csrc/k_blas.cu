@@ -48,6 +48,50 @@ __device__ __forceinline__ double2 block_sum(double2 v)
   return v;
 }
 
+// block_sum of one or two values per thread into memory. Same additions in the same tree, but a
+// lane adds one component only: the halves (quarters) of a warp trade the components they drop
+// for the partner's. An addition of a warp takes the FP64 unit 16 cycles, and a block of a short
+// chunk is bound by them: 43 or 51 additions instead of 90 or 180 (6 systems of 84^3 cells: a
+// complex64 dot 50 -> 37 us, two at once 83 -> 53, with the update of x and r 149 -> 121).
+__device__ __forceinline__ double add_down(double v, int o) { return __dadd_rn(v, __shfl_down_sync(0xffffffffu, v, o)); }
+__device__ __forceinline__ double trade(double lo, double hi, int bit)
+{
+  const bool up = threadIdx.x & bit;
+  return __dadd_rn(up ? hi : lo, __shfl_xor_sync(0xffffffffu, up ? lo : hi, bit));
+}
+__device__ __forceinline__ void block_sum_to(double2 v, double2* dst)
+{
+  __shared__ double red[2][DOT_THREADS / 32];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  double s = trade(v.x, v.y, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) s = add_down(s, o);
+  if ((l & 15) == 0) red[l >> 4][w] = s;
+  __syncthreads();
+  if (w == 0) {
+    s = red[l >> 4][l & 7];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s = add_down(s, o);
+    if ((l & 15) == 0) (&dst->x)[l >> 4] = s;
+  }
+}
+__device__ __forceinline__ void block_sum_to(double2 v1, double2 v2, double2* dst1, double2* dst2)
+{
+  __shared__ double red[4][DOT_THREADS / 32];  // x1, x2, y1, y2
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  double s = trade(trade(v1.x, v1.y, 16), trade(v2.x, v2.y, 16), 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) s = add_down(s, o);
+  if ((l & 7) == 0) red[l >> 3][w] = s;
+  __syncthreads();
+  if (w == 0) {
+    s = red[l >> 3][l & 7];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s = add_down(s, o);
+    if ((l & 7) == 0) (&(l & 8 ? dst2 : dst1)->x)[l >> 4] = s;
+  }
+}
+
 // partial[slot][blk] = sum over the block's chunk of a*conj(b), Acc's way
 template <class P, class Acc>
 __global__ void __launch_bounds__(DOT_THREADS)
@@ -61,9 +105,9 @@ k_dot_partial(const typename P::C* __restrict__ A, const typename P::C* __restri
   const long chunk = (n + nblk - 1) / nblk;
   const long beg = (long)blockIdx.x * chunk, end = min(n, beg + chunk);
   Acc d;
+#pragma unroll 4
   for (long q = beg + threadIdx.x; q < end; q += DOT_THREADS) d.add(a[q], b[q]);
-  const double2 acc = block_sum(d.value());
-  if (threadIdx.x == 0) partial[(size_t)slot * nblk + blockIdx.x] = acc;
+  block_sum_to(d.value(), partial + (size_t)slot * nblk + blockIdx.x);
 }
 
 // The whole dot product of a short vector (nblk <= DOT_CLUSTER) in one launch. The warps of
@@ -133,12 +177,8 @@ k_dot2_partial(const typename P::C* __restrict__ A1, const typename P::C* __rest
     d1.add(A1[so + q], B1[so + q]);
     d2.add(A2[so + q], B2[so + q]);
   }
-  const double2 acc1 = block_sum(d1.value());
-  const double2 acc2 = block_sum(d2.value());
-  if (threadIdx.x == 0) {
-    partial[(size_t)slot * nblk + blockIdx.x] = acc1;
-    partial[(size_t)(gridDim.y + slot) * nblk + blockIdx.x] = acc2;
-  }
+  block_sum_to(d1.value(), d2.value(), partial + (size_t)slot * nblk + blockIdx.x,
+               partial + (size_t)(gridDim.y + slot) * nblk + blockIdx.x);
 }
 
 __global__ void k_dot_final(const double2* __restrict__ partial, int nblk, double2* __restrict__ out)
@@ -249,12 +289,8 @@ k_xr_dot2(long n, const int* __restrict__ sys_list, const KrylovScalars* __restr
     d1.add(rv, rv);
     d2.add(rv, r0[so + q]);
   }
-  const double2 acc1 = block_sum(d1.value());
-  const double2 acc2 = block_sum(d2.value());
-  if (threadIdx.x == 0) {
-    partial[(size_t)slot * nblk + blockIdx.x] = acc1;
-    partial[(size_t)(gridDim.y + slot) * nblk + blockIdx.x] = acc2;
-  }
+  block_sum_to(d1.value(), d2.value(), partial + (size_t)slot * nblk + blockIdx.x,
+               partial + (size_t)(gridDim.y + slot) * nblk + blockIdx.x);
 }
 
 template <class P>
@@ -295,8 +331,7 @@ k_res_norm(long n, const int* __restrict__ sys_list, const double2* __restrict__
     x = fma(v.x, v.x, x);
     y = fma(v.y, v.y, y);
   }
-  const double2 acc = block_sum(make_double2(x + y, 0.));
-  if (threadIdx.x == 0) partial[(size_t)slot * nblk + blockIdx.x] = acc;
+  block_sum_to(make_double2(x + y, 0.), partial + (size_t)slot * nblk + blockIdx.x);
 }
 
 void launch_res_norm(long n, int nslot, const int* sys_list, const double2* b, const double2* w, double2* r,
