@@ -58,13 +58,14 @@ template <class P>
 void launch_air_scatter(const AirP<P>& a, const typename P::C* K2, typename P::C* ghx, typename P::C* ghy,
                         int nslot, cudaStream_t st);
 
-// complex64 airwave in three kernels of its own (k_airwave32.cu); the filters transposed
+// airwave by line transforms, three kernels (k_airlines.cu); complex64's filters transposed
 // ([N1][N2]), T: nslot * n2 * N1, T12: nslot * (2 n2 + 1) * N1, tw: air_twiddles(N1)
-bool airwave32_fits(int n1, int n2, int N1, int N2);
-std::vector<float2> air_twiddles(int N);
-void launch_airwave32(const GridP<F32>& g, const AirP<F32>& a, const SysScal<F32>* scal, const float2* X,
-                      const int* sys_list, const float2* tw, float2* T, float2* T12, float2* ghx, float2* ghy,
-                      int nslot, cudaStream_t st);
+bool air_lines_fit(int n1, int n2, int N1, int N2);
+std::vector<double2> air_twiddles(int N);
+template <class P>
+void launch_air_lines(const GridP<P>& g, const AirP<P>& a, const SysScal<P>* scal, const typename P::C* X,
+                      const int* sys_list, const typename P::C* tw, typename P::C* T,
+                      typename P::C* T12, typename P::C* ghx, typename P::C* ghy, int nslot, cudaStream_t st);
 
 // ---------------------------------------------------------------- LU-SGS / A-phi
 // A component sweep over one wavefront diagonal. The sweep grid has nK planes

@@ -162,7 +162,7 @@ Model::Model(const csem_grid* gp, int airbc_, int fvm_)
     back(G.x2, n2 + 1, G.d2fft);
     // the line transforms take a node past the uniform grid as zero, k_air_scatter the next
     // row's first: the same where its weight is rounding
-    air_lines = airwave32_fits(n1, n2, N1, N2);
+    air_lines = air_lines_fit(n1, n2, N1, N2);
     for (size_t q = back0; q < ih.size(); q++)
       if (ih[q] < 0 || ih[q] >= N1 || (ih[q] == N1 - 1 && fabs(wh[q]) > 1e-9)) air_lines = false;
     upload(air_i, ih);
@@ -179,7 +179,13 @@ Model::Model(const csem_grid* gp, int airbc_, int fvm_)
       f32[t] = make_float2((float)f64[q].x, (float)f64[q].y);
       f32[NN + t] = make_float2((float)f64[NN + q].x, (float)f64[NN + q].y);
     }
-    if (air_lines) upload(air_tw, air_twiddles(N1));
+    if (air_lines) {
+      const std::vector<double2> tw = air_twiddles(N1);
+      std::vector<float2> tf;
+      for (const double2& t : tw) tf.push_back(make_float2((float)t.x, (float)t.y));
+      upload(air_tw64, tw);
+      upload(air_tw, tf);
+    }
     upload(sH64, f64);
     upload(sH32, f32);
     auto afill = [&](auto& a, auto* w, auto* sh) {
@@ -366,13 +372,10 @@ bool Ops<P>::apply_A(const C* X, C* Y, int nslot, const int* sys_list, const Sys
   if (m->airbc) {
     const AirP<P>& a = m->air<P>();
     ProfScope air(P::exact ? PROF_AIR64 : PROF_AIR32, st, nslot);
-    bool lines = false;
-    if constexpr (!P::exact) {
-      if ((lines = m->air_lines)) {
-        launch_airwave32(g, a, sc, X, sys_list, m->air_tw.template as<C>(), K.as<C>(), K2.as<C>(), ghx.as<C>(),
-                         ghy.as<C>(), nslot, st);
-      }
-    }
+    const bool lines = m->air_lines && (!P::exact || quick_stencil);
+    if (lines)
+      launch_air_lines<P>(g, a, sc, X, sys_list, (P::exact ? m->air_tw64 : m->air_tw).template as<C>(),
+                          K.as<C>(), K2.as<C>(), ghx.as<C>(), ghy.as<C>(), nslot, st);
     if (!lines) {
       launch_hz0<P>(g, sc, X, hz0.as<C>(), nslot, sys_list, st);
       launch_air_gather<P>(a, hz0.as<C>(), K.as<C>(), nslot, st);

@@ -59,14 +59,14 @@ class Model {
   float rho_water;
   int N1 = 0, N2 = 0;  // airwave grid
   // device data
-  DevBuf d64, d32, q64, s64, s32, x64, air_i, air_w64, air_w32, sH64, sH32, air_tw;
+  DevBuf d64, d32, q64, s64, s32, x64, air_i, air_w64, air_w32, sH64, sH32, air_tw, air_tw64;
   GridP<F64> g64;  // operator view (kstart shift applied inside kernels)
   GridP<F32> g32;
   AirP<F64> a64;
   AirP<F32> a32;
   AcqGrid acq;
-  // complex64 airwave by k_airwave32.cu (sH32 is then transposed, air_tw its twiddles) instead
-  // of cuFFT
+  // the airwave of complex64 and of quick complex128 by k_airlines.cu instead of cuFFT (sH32 is
+  // then transposed, air_tw and air_tw64 hold the twiddles)
   bool air_lines = false;
   // cuFFT plans of this model's airwave grid (one set per model: a plan is bound to one
   // stream at a time, and contexts may run on different host threads)
