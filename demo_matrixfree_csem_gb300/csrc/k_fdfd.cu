@@ -10,6 +10,7 @@
 // With the airwave boundary (airbc=1) the k=0 rows of bx/by use the ghost fields
 // Hx(z=-dz/2), Hy(z=-dz/2) that the airwave pipeline derives from Hz(z=0)
 // (fdfd.c:151-172); k_hz0 provides that Hz plane.
+#include <type_traits>
 #include "csem_cuda.cuh"
 #include "engine.h"
 
@@ -49,8 +50,7 @@ __device__ __forceinline__ void h_at(const GridP<P>& g, const typename P::C* __r
 // Hy and Hz from the previous lane, and the j-1 neighbours of Hx and Hz from the
 // previous warp through shared memory (double-buffered by plane parity, one barrier per
 // plane). Its column's spacings stay in registers and its element offsets advance by one
-// plane stride per plane; the plane's spacings are uniform loads. H is evaluated exactly
-// as in h_at, so complex128 results keep their bits.
+// plane stride per plane; the plane's spacings are uniform loads.
 template <class P, int BY>
 __global__ void __launch_bounds__(32 * (BY + 1), 1)
 k_fdfd(GridP<P> g, const SysScal<P>* __restrict__ scal, const typename P::C* __restrict__ X,
@@ -126,89 +126,99 @@ k_fdfd(GridP<P> g, const SysScal<P>* __restrict__ scal, const typename P::C* __r
     return p;
   };
   PlaneIn nxt = load_plane(kb, oEx, oEy, oEz);
-  for (int k = kb; k < ke; k++, oEx += sEx, oEy += sEy, oEz += sEz) {
-    const int kf = k + ks;
-    const int pb = k & 1;
-    const bool kin = k < n3;
-    const PlaneIn cur = nxt;
-    if (k + 1 < ke) nxt = load_plane(k + 1, oEx + sEx, oEy + sEy, oEz + sEz);
-    const R d3s = g.d3s[kf], r3s = g.r3s[kf], d3 = g.d3[kf], r3 = g.r3[kf];
-    const C ez = cur.ez, ezj = cur.ezj, exj = cur.exj, ex1 = cur.ex1, ey1 = cur.ey1;
-    C ezi, eyi;  // Ez(k, j, i+1), Ey(k, j, i+1): the next lane's, loaded by the last lane
-    ezi.x = __shfl_down_sync(0xffffffffu, ez.x, 1);
-    ezi.y = __shfl_down_sync(0xffffffffu, ez.y, 1);
-    eyi.x = __shfl_down_sync(0xffffffffu, eyk.x, 1);
-    eyi.y = __shfl_down_sync(0xffffffffu, eyk.y, 1);
-    if (lane == 31) {
-      ezi = hasEx && kin ? Ez[oEz + 1] : z;
-      eyi = hasExj ? Ey[oEy + 1] : z;
-    }
-    // H at (k, j, i), the operations of h_at
-    hx = hy = hz = z;
-    if (hasEy && kin) {
-      C t1 = cdivs<P>(csub<P>(ezj, ez), d2s, r2s);
-      C t2 = cdivs<P>(csub<P>(ey1, eyk), d3s, r3s);
-      hx = cmul<P>(csub<P>(t1, t2), iwmu);
-    }
-    if (hasEx && kin) {
-      C t1 = cdivs<P>(csub<P>(ex1, exk), d3s, r3s);
-      C t2 = cdivs<P>(csub<P>(ezi, ez), d1s, r1s);
-      hy = cmul<P>(csub<P>(t1, t2), iwmu);
-    }
-    if (hasExj) {
-      C t1 = cdivs<P>(csub<P>(eyi, eyk), d1s, r1s);
-      C t2 = cdivs<P>(csub<P>(exj, exk), d2s, r2s);
-      hz = cmul<P>(csub<P>(t1, t2), iwmu);
-    }
-    sHx[pb][w][lane] = hx;
-    sHz[pb][w][lane] = hz;
-    C hyl, hzl;  // Hy(k, j, i-1), Hz(k, j, i-1) from the previous lane
-    hyl.x = __shfl_up_sync(0xffffffffu, hy.x, 1);
-    hyl.y = __shfl_up_sync(0xffffffffu, hy.y, 1);
-    hzl.x = __shfl_up_sync(0xffffffffu, hz.x, 1);
-    hzl.y = __shfl_up_sync(0xffffffffu, hz.y, 1);
-    __syncthreads();
-    if (interior) {
-      const C hxd = sHx[pb][w - 1][lane], hzd = sHz[pb][w - 1][lane];  // at j-1
-      const bool kxy = (k >= 1 && k <= n3 - 1) || (k == 0 && g.airbc);
-      if (outX) {  // bx
-        C r = z;
-        if (inX && kxy) {
-          C hyb = k >= 1 ? pHy : ghy[i + (long)n1 * j];
-          C t1 = cdivs<P>(csub<P>(hz, hzd), d2, r2);
-          C t2 = cdivs<P>(csub<P>(hy, hyb), d3, r3);
-          r = csub<P>(csub<P>(t1, t2), rmul<P>(cur.s1, exk));
-          if (g.fvm) r = cmul<P>(r, rmul<P>(P::mul(P::mul(d1s, d2), d3), iom));
-        }
-        bx[oEx] = r;
+  // imag: 1 / (i w mu0) is imaginary, as for real frequencies; it goes into the spacings'
+  // reciprocals, and H = i t: 54 FP64 operations a cell instead of 66, which bind this kernel (24
+  // systems of 3.7 M cells: 15.3 -> 14.3 ms with 8 rows a tile)
+  auto march = [&](auto imag) {
+    constexpr bool IMAG = decltype(imag)::value;
+    auto times = [&](C t) { return IMAG ? P::mk(-t.y, t.x) : cmul<P>(t, iwmu); };
+    const R q1s = IMAG ? r1s * iwmu.y : r1s, q2s = IMAG ? r2s * iwmu.y : r2s;
+    for (int k = kb; k < ke; k++, oEx += sEx, oEy += sEy, oEz += sEz) {
+      const int kf = k + ks;
+      const int pb = k & 1;
+      const bool kin = k < n3;
+      const PlaneIn cur = nxt;
+      if (k + 1 < ke) nxt = load_plane(k + 1, oEx + sEx, oEy + sEy, oEz + sEz);
+      const R d3s = g.d3s[kf], q3s = IMAG ? g.r3s[kf] * iwmu.y : g.r3s[kf], d3 = g.d3[kf], r3 = g.r3[kf];
+      const C ez = cur.ez, ezj = cur.ezj, exj = cur.exj, ex1 = cur.ex1, ey1 = cur.ey1;
+      C ezi, eyi;  // Ez(k, j, i+1), Ey(k, j, i+1): the next lane's, loaded by the last lane
+      ezi.x = __shfl_down_sync(0xffffffffu, ez.x, 1);
+      ezi.y = __shfl_down_sync(0xffffffffu, ez.y, 1);
+      eyi.x = __shfl_down_sync(0xffffffffu, eyk.x, 1);
+      eyi.y = __shfl_down_sync(0xffffffffu, eyk.y, 1);
+      if (lane == 31) {
+        ezi = hasEx && kin ? Ez[oEz + 1] : z;
+        eyi = hasExj ? Ey[oEy + 1] : z;
       }
-      if (outY) {  // by
-        C r = z;
-        if (inY && kxy) {
-          C hxb = k >= 1 ? pHx : ghx[i + (long)(n1 + 1) * j];
-          C t1 = cdivs<P>(csub<P>(hx, hxb), d3, r3);
-          C t2 = cdivs<P>(csub<P>(hz, hzl), d1, r1);
-          r = csub<P>(csub<P>(t1, t2), rmul<P>(cur.s2, eyk));
-          if (g.fvm) r = cmul<P>(r, rmul<P>(P::mul(P::mul(d1, d2s), d3), iom));
-        }
-        by[oEy] = r;
+      // H at (k, j, i), as in h_at
+      hx = hy = hz = z;
+      if (hasEy && kin) {
+        C t1 = cdivs<P>(csub<P>(ezj, ez), d2s, q2s);
+        C t2 = cdivs<P>(csub<P>(ey1, eyk), d3s, q3s);
+        hx = times(csub<P>(t1, t2));
       }
-      if (outZ && kin) {  // bz
-        C r = z;
-        if (inZ) {
-          C t1 = cdivs<P>(csub<P>(hy, hyl), d1, r1);
-          C t2 = cdivs<P>(csub<P>(hx, hxd), d2, r2);
-          r = csub<P>(csub<P>(t1, t2), rmul<P>(cur.s3, ez));
-          if (g.fvm) r = cmul<P>(r, rmul<P>(P::mul(P::mul(d1, d2), d3s), iom));
-        }
-        bz[oEz] = r;
+      if (hasEx && kin) {
+        C t1 = cdivs<P>(csub<P>(ex1, exk), d3s, q3s);
+        C t2 = cdivs<P>(csub<P>(ezi, ez), d1s, q1s);
+        hy = times(csub<P>(t1, t2));
       }
+      if (hasExj) {
+        C t1 = cdivs<P>(csub<P>(eyi, eyk), d1s, q1s);
+        C t2 = cdivs<P>(csub<P>(exj, exk), d2s, q2s);
+        hz = times(csub<P>(t1, t2));
+      }
+      sHx[pb][w][lane] = hx;
+      sHz[pb][w][lane] = hz;
+      C hyl, hzl;  // Hy(k, j, i-1), Hz(k, j, i-1) from the previous lane
+      hyl.x = __shfl_up_sync(0xffffffffu, hy.x, 1);
+      hyl.y = __shfl_up_sync(0xffffffffu, hy.y, 1);
+      hzl.x = __shfl_up_sync(0xffffffffu, hz.x, 1);
+      hzl.y = __shfl_up_sync(0xffffffffu, hz.y, 1);
+      __syncthreads();
+      if (interior) {
+        const C hxd = sHx[pb][w - 1][lane], hzd = sHz[pb][w - 1][lane];  // at j-1
+        const bool kxy = (k >= 1 && k <= n3 - 1) || (k == 0 && g.airbc);
+        if (outX) {  // bx
+          C r = z;
+          if (inX && kxy) {
+            C hyb = k >= 1 ? pHy : ghy[i + (long)n1 * j];
+            C t1 = cdivs<P>(csub<P>(hz, hzd), d2, r2);
+            C t2 = cdivs<P>(csub<P>(hy, hyb), d3, r3);
+            r = csub<P>(csub<P>(t1, t2), rmul<P>(cur.s1, exk));
+            if (g.fvm) r = cmul<P>(r, rmul<P>(P::mul(P::mul(d1s, d2), d3), iom));
+          }
+          bx[oEx] = r;
+        }
+        if (outY) {  // by
+          C r = z;
+          if (inY && kxy) {
+            C hxb = k >= 1 ? pHx : ghx[i + (long)(n1 + 1) * j];
+            C t1 = cdivs<P>(csub<P>(hx, hxb), d3, r3);
+            C t2 = cdivs<P>(csub<P>(hz, hzl), d1, r1);
+            r = csub<P>(csub<P>(t1, t2), rmul<P>(cur.s2, eyk));
+            if (g.fvm) r = cmul<P>(r, rmul<P>(P::mul(P::mul(d1, d2s), d3), iom));
+          }
+          by[oEy] = r;
+        }
+        if (outZ && kin) {  // bz
+          C r = z;
+          if (inZ) {
+            C t1 = cdivs<P>(csub<P>(hy, hyl), d1, r1);
+            C t2 = cdivs<P>(csub<P>(hx, hxd), d2, r2);
+            r = csub<P>(csub<P>(t1, t2), rmul<P>(cur.s3, ez));
+            if (g.fvm) r = cmul<P>(r, rmul<P>(P::mul(P::mul(d1, d2), d3s), iom));
+          }
+          bz[oEz] = r;
+        }
+      }
+      pHx = hx;
+      pHy = hy;
+      exk = ex1;
+      eyk = ey1;
     }
-    pHx = hx;
-    pHy = hy;
-    exk = ex1;
-    eyk = ey1;
-  }
+  };
+  if (iwmu.x == 0) march(std::true_type());
+  else march(std::false_type());
 }
 
 // Hz on the plane k=0 (operator grid) for the airwave: out[sys][j][i], i<n1, j<n2
@@ -283,9 +293,10 @@ void launch_fdfd(const GridP<P>& g, const SysScal<P>* scal, const typename P::C*
                  const typename P::C* ghx, const typename P::C* ghy, int nsys, const int* sys_list,
                  cudaStream_t st, int by, int ctas_per_sm)
 {
+  // 16 rows but where 4 are asked for: of the FP64 operations that bind it the halo takes 9% (8
+  // rows: 14%, 12: 11%; 24 systems of 3.7 M cells 13.0, 14.3 and 13.2 ms, 4 rows 17.5)
   if (by == 4) launch_fdfd_by<P, 4>(g, scal, X, Y, ghx, ghy, nsys, sys_list, st, ctas_per_sm);
-  else if (by == 16) launch_fdfd_by<P, 16>(g, scal, X, Y, ghx, ghy, nsys, sys_list, st, ctas_per_sm);
-  else launch_fdfd_by<P, 8>(g, scal, X, Y, ghx, ghy, nsys, sys_list, st, ctas_per_sm);
+  else launch_fdfd_by<P, 16>(g, scal, X, Y, ghx, ghy, nsys, sys_list, st, ctas_per_sm);
 }
 
 template <class P>
