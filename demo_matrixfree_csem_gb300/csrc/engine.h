@@ -135,6 +135,8 @@ void launch_line_pass(const SweepP<F32>& s, int comp, bool fwd, int nslot, float
                       const int* groups, int ngroups, cudaStream_t st);
 // zeros where the line sweeps read and never write (instead of clearing Y and CAP)
 void launch_line_bounds(const SweepP<F32>& s, int nslot, cudaStream_t st);
+// T = X + sigma grad v: A-phi's backward edge sweeps as LU-SGS's with this right-hand side
+void launch_aphi_rhs(const SweepP<F32>& s, float2* T, int nslot, cudaStream_t st);
 void launch_sweep_line(const SweepP<F32>& s, int comp, bool fwd, int nslot, const float2* SB, const float2* SW, long sbs,
                        const int* group_of, cudaStream_t st);
 bool sweep_line_fits(int n1, int n2, int nK);  // the rows' tables and edge columns fit shared memory

@@ -347,10 +347,10 @@ template <class P> Ops<P>::~Ops()
   if (aux) cudaStreamDestroy(aux);
 }
 
-template <class P> bool Ops<P>::line_fits() const
+template <class P> bool Ops<P>::line_fits(int nK) const
 {
   return !P::exact && split_sweeps && line_sweeps && pipelined_sweeps && !tiled_sweeps &&
-         sweep_line_fits(m->n1, m->n2, m->airbc ? m->n3f : m->n3);
+         sweep_line_fits(m->n1, m->n2, nK);
 }
 
 template <class P> int Ops<P>::split_ctas() const { return split_cap > 0 ? split_cap * sm_count() : 0; }
@@ -621,15 +621,34 @@ void Ops<P>::apply_aphi(const C* X, C* Y, int nslot, const int* sys_list, const 
   s.s33u = gu.s33;
   s.aphi_fix = aphi_fix ? 1 : 0;
   const int n1 = m->n1, n2 = m->n2, n3 = m->n3;
-  zero(Y, m->lE, nslot, sys_list);
+  const bool lines = line_fits(n3);
+  const long sbs = sweep_split_scratch(n1, n2, n3);
+  if constexpr (!P::exact) {
+    if (lines) {
+      if (sb.bytes < sizeof(float4) * (size_t)sbs * nmax) sb.alloc(sizeof(float4) * (size_t)sbs * nmax);
+      if (!rhs.p) rhs.alloc(sizeof(C) * (size_t)m->lE * nmax);
+      launch_line_bounds(s, nslot, st);
+    }
+  }
+  if (!lines) zero(Y, m->lE, nslot, sys_list);
   launch_aphi_div<P>(s, BV.as<C>(), nslot, st);
   CSEM_CUDA_TRY(cudaMemsetAsync(V.p, 0, sizeof(C) * (size_t)m->lv * nslot, st));
   if constexpr (P::exact) {
     if (pipelined_sweeps) diag_table(s, nslot);
   }
-  // an edge sweep in one launch where the complex128 pipeline takes it, else by diagonals
+  // an edge sweep in one launch where the complex128 pipeline takes it, complex64 as LU-SGS's by
+  // lines, else by diagonals
   auto edges = [&](int comp, bool fwd) {
-    if constexpr (P::exact) {
+    if constexpr (!P::exact) {
+      if (lines) {
+        SweepP<P> e = s;
+        if (!fwd) e.X = rhs.as<C>();
+        float2 *SB = sb.as<float2>(), *SW = SB + (size_t)nslot * sbs;
+        launch_line_pass(e, comp, fwd, nslot, SB, SW, sbs, nullptr, 0, st);
+        launch_sweep_line(e, comp, fwd, nslot, SB, SW, sbs, nullptr, st);
+        return;
+      }
+    } else {
       if (pipelined_sweeps && sweep_pipelined_fits(comp, n1, n2, n3)) {
         launch_sweep64(s, comp, fwd, true, nslot, tab.p, st);
         return;
@@ -651,6 +670,9 @@ void Ops<P>::apply_aphi(const C* X, C* Y, int nslot, const int* sys_list, const 
   };
   for (int t = 3; t < 3 + np; t++) nodes(t);
   for (int t = 2 + np; t >= 3; t--) nodes(-t);
+  if constexpr (!P::exact) {
+    if (lines) launch_aphi_rhs(s, rhs.as<C>(), nslot, st);
+  }
   for (int comp = 2; comp >= 0; comp--) edges(comp, false);
   launch_aphi_grad<P>(s, V.as<C>(), nslot, st);
 }

@@ -125,7 +125,7 @@ class Ops {
   Model* m;
   int nmax;
   cudaStream_t st;
-  DevBuf hz0, K, K2, ghx, ghy, cap, V, BV, scal, sb, tab;
+  DevBuf hz0, K, K2, ghx, ghy, cap, V, BV, scal, sb, tab, rhs;
   FftPlans* fft;
   // LU-SGS sweeps: true = one pipelined-warp launch per component sweep (k_lusgs2.cu),
   // false = one launch per wavefront diagonal (k_lusgs.cu); both give identical results
@@ -143,7 +143,8 @@ class Ops {
   bool split_sweeps = true;
   // split sweeps with a warp per line in the row pipeline's place (k_lusgs6.cu), on one stream
   bool line_sweeps = true;
-  bool line_fits() const;  // they are on and take this grid
+  bool line_fits(int nK) const;  // they are on and take this grid (nK: its planes)
+  bool line_fits() const { return line_fits(m->airbc ? m->n3f : m->n3); }
   // whether the caller should number the groups within two halves of the slots
   bool halves() const { return split_sweeps && split_overlap && !line_fits(); }
   // split sweeps on two halves of the slots, one on `aux`, so that one half's passes can

@@ -359,6 +359,36 @@ __global__ void __launch_bounds__(128) k_line_bounds(SweepP<F32> s)
     for (int q = threadIdx.x; q < H; q += 128) p[(long)q * W] = p[(long)q * W + n1] = z;
 }
 
+// A-phi's backward edge sweeps as LU-SGS's: their extra term, sigma grad v (fdfd.c:735-790, times
+// the cell's volume and i omega in finite volumes), goes into the right-hand side T, [slot's
+// system][lE]. grid (edges, slots)
+__global__ void __launch_bounds__(256) k_aphi_rhs(SweepP<F32> s, C* T)
+{
+  const GridP<F32>& g = s.g;
+  const int n1 = g.n1, n2 = g.n2, n3 = g.n3, L1 = n1 + 1, slot = blockIdx.y;
+  const long q = (long)blockIdx.x * 256 + threadIdx.x;
+  if (q >= g.lE) return;
+  const int sys = s.sys_list ? s.sys_list[slot] : slot;
+  const C* v = s.V + (size_t)slot * s.lv;
+  const int c = q < g.lEx ? 0 : (q < g.lEx + g.lEy ? 1 : 2);
+  const unsigned r = (unsigned)(q - (c == 0 ? 0 : (c == 1 ? g.lEx : g.lEx + g.lEy)));
+  const unsigned W = c == 0 ? n1 : L1, H = c == 1 ? n2 : n2 + 1;
+  const int i = r % W, j = r / W % H, k = r / (W * H);
+  C t = ro(s.X + (size_t)sys * g.lE + q);
+  if ((c == 0 || (i >= 1 && i < n1)) && (c == 1 || (j >= 1 && j < n2)) && (c == 2 || (k >= 1 && k < n3))) {
+    const long n = ix3(n1, n2, k, j, i);
+    const C hi = ro(v + n + (c == 0 ? 1 : (c == 1 ? L1 : (long)L1 * (n2 + 1)))), lo = ro(v + n);
+    const float f = (c == 0 ? ro(g.s11 + r) * ro(g.r1s + i) : (c == 1 ? ro(g.s22 + r) * ro(g.r2s + j) : ro(g.s33 + r) * ro(g.r3s + k)));
+    C e = make_float2(f * (hi.x - lo.x), f * (hi.y - lo.y));
+    if (g.fvm) {
+      const SysScal<F32> sc = s.scal[sys];
+      e = mul32(e, scl32(ro(g.d1s + i) * ro(g.d2 + j) * ro(g.d3 + k), sc.iom));
+    }
+    t = make_float2(t.x + e.x, t.y + e.y);
+  }
+  T[(size_t)sys * g.lE + q] = t;
+}
+
 template <int COMP, bool FWD, int LINES, int CH>
 __global__ void __launch_bounds__(64 * LINES) k_line32(SweepP<F32> s, const float2* SB, const float2* SW,
                                                                         long sbs, const int* group_of, int groups_per_slot)
@@ -632,6 +662,11 @@ bool sweep_line_fits(int n1, int n2, int nK)
 void launch_line_bounds(const SweepP<F32>& s, int nslot, cudaStream_t st)
 {
   count_launch(), k_line_bounds<<<dim3(s.nK + 1, 3, nslot), 128, 0, st>>>(s);
+}
+
+void launch_aphi_rhs(const SweepP<F32>& s, float2* T, int nslot, cudaStream_t st)
+{
+  count_launch(), k_aphi_rhs<<<dim3((unsigned)((s.g.lE + 255) / 256), nslot), 256, 0, st>>>(s, T);
 }
 
 void launch_line_pass(const SweepP<F32>& s, int comp, bool fwd, int nslot, float2* SB, float2* SW, long sbs,
