@@ -12,9 +12,9 @@
 // The pass: a thread per point, which forms 1/aii and w once for its frequency's systems. A
 // point's operands lie at the same offsets in every system, so they are formed once, too,
 // relative to the planes k and k-1 (k+1 for Ez), each in y or in the cap. Ex's lines are
-// i, the axis its operands are contiguous on, so 32 x 32 tiles turn in shared memory. A thread
+// i, the axis its operands are contiguous on, so 32 x 16 tiles turn in shared memory. A thread
 // forms two points, for the loads in flight; Ey's and Ez's are of neighbouring rows j and share
-// some (11 -> 9 or 10 a point). 64 registers, for 32 warps an SM.
+// some (11 -> 9 or 10 a point). 64 registers (Ex 80), for 32 warps an SM (24).
 //
 // The chain: a warp owns one line and works through its march in strips of 32 positions, lane t on
 // position t of the strip, over all rows of the strip before the next strip. Lane t runs t
@@ -36,9 +36,9 @@
 // The thread-per-row pipelines (k_sweep_ex32s, k_sweep_eyz32s, lusgs_split 1) read one 16-byte
 // entry per row and lane, 20 sectors a request, and join a line's warps by barriers at every
 // step. Per application, them, this with one warp to a line and one point to a pass's thread, and
-// this, one context: 200 x 140 x 140 cells, 48 systems 23.3, 14.6, 13.9 ms, 16 systems 8.02,
-// 5.30, 4.81, 3 systems 2.11, 1.40, 1.16; 84^3 cells, 6 systems 0.86, 0.51, 0.42; 81 x 73 x 67
-// cells, 3 systems at 3 frequencies 0.51, 0.35, 0.27. The pass takes 60% of it, at 60% of the
+// this, one context: 200 x 140 x 140 cells, 48 systems 23.3, 14.6, 12.8 ms, 16 systems 8.02,
+// 5.30, 4.44, 3 systems 2.11, 1.40, 1.08; 84^3 cells, 6 systems 0.86, 0.51, 0.39; 81 x 73 x 67
+// cells, 3 systems at 3 frequencies 0.51, 0.35, 0.25. The pass takes 60% of it, at 60% of the
 // DRAM rate, bound by its loads' latency; the chain runs at 50% (large batches: 7 or 8 lines on
 // an SM by its shared memory, and its load and store unit) or is bound by its steps' latency, 640
 // cycles for 8 rows (small ones).
@@ -255,12 +255,14 @@ __global__ void __launch_bounds__(32 * PASS_WARPS, 16)
   for (int q = 0; q < mem.n; q++) form(q, load(q));
 }
 
-// Ex: a CTA forms 32 i x a strip's 32 positions j, along i, and stores them along j.
-// grid (i tiles x groups, strips, k)
+// Ex: a CTA forms 32 i x half a strip's 16 positions j, along i, and stores them along j, 128 bytes
+// a line. 3 CTAs with 80 registers: a barrier per system stops a third of an SM (an application, 48
+// systems of 200 x 140 x 140 cells: 12.78 ms; 2 CTAs of whole strips, 64 registers and spills,
+// 12.92; 4 of half strips 12.85, 5 13.63). grid (i tiles x groups, half strips, k)
 template <bool FWD, int NS>
-__global__ void __launch_bounds__(512, 2) k_line_pass_ex(SweepP<F32> s, float2* SB, float2* SW, long sbs, int nti, const int* groups)
+__global__ void __launch_bounds__(256, 3) k_line_pass_ex(SweepP<F32> s, float2* SB, float2* SW, long sbs, int nti, const int* groups)
 {
-  __shared__ C tiles[2][32][33];  // one is written while the other's values go out
+  __shared__ C tiles[2][32][17];  // one is written while the other's values go out
   const GridP<F32>& g = s.g;
   const int n1 = g.n1, n2 = g.n2, L1 = n1 + 1;
   const int grp = blockIdx.x / nti, i0 = (blockIdx.x - grp * nti) * 32, k = 1 + blockIdx.z;
@@ -277,7 +279,7 @@ __global__ void __launch_bounds__(512, 2) k_line_pass_ex(SweepP<F32> s, float2* 
   unsigned ox[2], oy[2], oz[2], ozm[2], oxm[2];
 #pragma unroll
   for (int a = 0; a < 2; a++) {
-    const int st = 32 * blockIdx.y + ty + 16 * a, j = FWD ? min(1 + st, M) : max(M - st, 1);  // (past the last position: it again)
+    const int st = 16 * blockIdx.y + ty + 8 * a, j = FWD ? min(1 + st, M) : max(M - st, 1);  // (past the last position: it again)
     const Ax<F32> Y = axis<F32>(g.d2, g.d2s, g.r2, g.r2s, j);
     const float gg = (Y.rs + Y.rsm) * Y.r + (Z.rs + Z.rsm) * Z.r;  // geo(Y, Z)
     cf[a] = lin_coef(sc, g.fvm, gg, ro(g.s11 + ix1(n1, n2, k, j, i)), xds * Y.d * Z.d);
@@ -288,14 +290,15 @@ __global__ void __launch_bounds__(512, 2) k_line_pass_ex(SweepP<F32> s, float2* 
     oy[a] = 8u * (unsigned)(plane(s, 1, k, upA) + (long)j * L1 + i);
     oz[a] = 8u * (unsigned)(plane(s, 2, k, upA) + (long)j * L1 + i);
     ozm[a] = 8u * (unsigned)(plane(s, 2, k - 1, upB) + (long)j * L1 + i);
-    tiles[1][tx][ty + 16 * a] = cf[a].w;
+    tiles[1][tx][ty + 8 * a] = cf[a].w;
   }
-  const size_t e0 = line_entry(S, Rp, i0 + ty, 32 * blockIdx.y + tx, FWD ? k - 1 : R - k), e1 = line_entry(S, Rp, 16, 0, 0);
-  const bool w0 = i0 + ty < n1, w1 = i0 + ty + 16 < n1;
-  auto turn = [&](C(*tile)[33], C* out) {
+  const int sp = threadIdx.x & 15, sl = threadIdx.x >> 4;
+  const size_t e0 = line_entry(S, Rp, i0 + sl, 16 * blockIdx.y + sp, FWD ? k - 1 : R - k), e1 = line_entry(S, Rp, 16, 0, 0);
+  const bool w0 = i0 + sl < n1, w1 = i0 + sl + 16 < n1;
+  auto turn = [&](C(*tile)[17], C* out) {
     __syncthreads();
-    if (w0) out[e0] = tile[ty][tx];
-    if (w1) out[e0 + e1] = tile[ty + 16][tx];
+    if (w0) out[e0] = tile[sl][sp];
+    if (w1) out[e0 + e1] = tile[sl + 16][sp];
   };
   turn(tiles[1], SW + (size_t)grp * sbs);
   const C z = make_float2(0.f, 0.f);
@@ -319,7 +322,7 @@ __global__ void __launch_bounds__(512, 2) k_line_pass_ex(SweepP<F32> s, float2* 
   load(0);
 #pragma unroll 1
   for (int q = 0; q < mem.n; q++) {
-    C(*tile)[33] = tiles[q & 1];
+    C(*tile)[17] = tiles[q & 1];
 #pragma unroll
     for (int a = 0; a < 2; a++) {
       C kc = z;
@@ -329,7 +332,7 @@ __global__ void __launch_bounds__(512, 2) k_line_pass_ex(SweepP<F32> s, float2* 
         const C cross = scl32(xrs, make_float2(yr[a] * dy.x + Z.r * dz.x, yr[a] * dy.y + Z.r * dz.y));
         kc = sub32(make_float2(kj[a] * v[a].ej.x + kz * v[a].ek.x, kj[a] * v[a].ej.y + kz * v[a].ek.y), cross);
       }
-      tile[tx][ty + 16 * a] = lin_B(cf[a], g.fvm, v[a].b, kc);
+      tile[tx][ty + 8 * a] = lin_B(cf[a], g.fvm, v[a].b, kc);
     }
     if (q + 1 < mem.n) load(q + 1);  // in flight while this system's tile turns
     turn(tile, SB + (size_t)mem.slot_of(q) * sbs);
@@ -597,9 +600,9 @@ void launch_pass(const SweepP<F32>& s, int sets, float2* SB, float2* SW, long sb
   const int n1 = s.g.n1, n2 = s.g.n2, nK = s.nK;
   if constexpr (COMP == 0) {
     const int nti = (n1 + 32 - 1) / 32;
-    dim3 grd((unsigned)(nti * sets), (unsigned)line_strips(n2 - 1), (unsigned)(nK - 1));
+    dim3 grd((unsigned)(nti * sets), (unsigned)(2 * line_strips(n2 - 1)), (unsigned)(nK - 1));
     keep_l1<k_line_pass_ex<FWD, NS>>(PASS_SMEM);
-    count_launch(), k_line_pass_ex<FWD, NS><<<grd, 512, 0, st>>>(s, SB, SW, sbs, nti, groups);
+    count_launch(), k_line_pass_ex<FWD, NS><<<grd, 256, 0, st>>>(s, SB, SW, sbs, nti, groups);
   } else {
     const int js = COMP == 1 ? n2 : n2 - 1, ks = COMP == 1 ? nK - 1 : nK;
     dim3 grd((unsigned)(line_strips(n1 - 1) * sets), (unsigned)((js + 2 * PASS_WARPS - 1) / (2 * PASS_WARPS)), (unsigned)ks);
