@@ -1,7 +1,8 @@
-// Airwave top boundary (airbc_init_free.c:130-209): Hz(z=0) on the stretched grid is
-// interpolated onto a uniform n1fft x n2fft grid, Fourier transformed (cuFFT, batched
-// over systems), multiplied by the two upward-continuation filters sH1/sH2, inverse
-// transformed, normalised and interpolated back onto the staggered ghost nodes
+// Airwave top boundary (airbc_init_free.c:130-209) by two-dimensional transforms: the complex128
+// solver's, whose rounding decides its iterates, and sides that k_airlines.cu does not take.
+// Hz(z=0) on the stretched grid is interpolated onto a uniform n1fft x n2fft grid, Fourier
+// transformed (cuFFT, batched over systems), multiplied by the two upward-continuation filters
+// sH1/sH2, inverse transformed, normalised and interpolated back onto the staggered ghost nodes
 // Hx(z=-dz/2) [(n2) x (n1+1)] and Hy(z=-dz/2) [(n2+1) x n1].
 //
 // The back-interpolation may address one node past the uniform grid (the last

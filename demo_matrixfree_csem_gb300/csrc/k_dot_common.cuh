@@ -1,5 +1,5 @@
 // Deterministic dot-product accumulation shared by the vector kernels (k_blas.cu) and the
-// stencil's fused dot products (k_fdfd.cu): per-thread accumulators of a*conj(b) and a
+// stencil's fused dot products (k_fdfd32.cu): per-thread accumulators of a*conj(b) and a
 // fixed shuffle tree.
 #pragma once
 #include "csem_cuda.cuh"

@@ -1,4 +1,6 @@
-// y = A x: the staggered-grid curl-curl operator of fdfd_apply (fdfd.c:86-205).
+// y = A x: the staggered-grid curl-curl operator of fdfd_apply (fdfd.c:86-205), in quick complex128
+// (F64Q, the batched solver's outer residuals); complex64 has k_fdfd32.cu, the reference's bits
+// k_fdfd64.cu. And what the stencils share: Hz of the top plane and the launch shape.
 //
 // One CTA owns a 31 x BY tile of (i,j) columns plus a one-column and one-row halo on the
 // low sides (the halo threads only compute H) and marches a chunk of z-planes. At each

@@ -1,4 +1,6 @@
-// LU-SGS complex64 component sweeps split into a coalesced pass and a light sweep.
+// LU-SGS complex64 component sweeps split into a coalesced pass and a light sweep: lusgs_split 1,
+// for grids that the line sweeps (k_lusgs6.cu, the default) do not take, and a candidate of the
+// autotuner.
 //
 // In the linear form of the complex64 sweeps (k_sweep_common.cuh), a point's value is
 // v = B + w (gp prev + gn nb): prev and nb are the only values written during the sweep
