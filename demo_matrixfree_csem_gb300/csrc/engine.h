@@ -89,6 +89,24 @@ template <class P> struct SweepP {
   int aphi_fix;             // 1: node sweeps with the conductivity-weighted diagonal (not the reference's)
 };
 
+// A hyperplane |t| of A-phi's node sweep, launched to start while the one before it (t other than
+// 3, the first) still runs
+struct PlaneLaunch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at;
+  template <class P> PlaneLaunch(const SweepP<P>& s, int t, int nslot, cudaStream_t st)
+  {
+    cfg.gridDim = dim3((s.g.n1 - 1 + 31) / 32, (s.g.n2 - 1 + 3) / 4, nslot);
+    cfg.blockDim = dim3(32, 4);
+    cfg.stream = st;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = t == 3 ? 0 : 1;
+  }
+  PlaneLaunch(const PlaneLaunch&) = delete;  // (cfg points into it)
+};
+
 // one launch per complex64 component sweep (pipelined warps, k_lusgs2.cu)
 void launch_sweep_pipelined(const SweepP<F32>& s, int comp, bool fwd, int nslot, cudaStream_t st, int vw,
                             int lines_per_cta = 1);

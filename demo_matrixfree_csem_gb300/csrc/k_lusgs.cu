@@ -281,6 +281,7 @@ __global__ void k_aphi_phi(SweepP<P> s, typename P::C* __restrict__ VV, int t)
   const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
   const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
   const int k = t - i - j;
+  cudaTriggerProgrammaticLaunchCompletion();  // the next hyperplane's blocks may come in and wait
   if (i >= n1 || j >= n2 || k < 1 || k >= n3) return;
   C* v = VV + (size_t)slot * s.lv;
   const C* bv = s.BV + (size_t)slot * s.lv;
@@ -289,11 +290,6 @@ __global__ void k_aphi_phi(SweepP<P> s, typename P::C* __restrict__ VV, int t)
   const C* az = ay + g.lEy;
   const SysScal<P> sc = s.scal[sys];
   const C z = czero<P>();
-  const C vp = z;  // v(k,j,i) is zeroed before its own update
-  const C vip = FWD ? z : v[ixv(n1, n2, k, j, i + 1)], vim = v[ixv(n1, n2, k, j, i - 1)];
-  const C vjp = FWD ? z : v[ixv(n1, n2, k, j + 1, i)], vjm = v[ixv(n1, n2, k, j - 1, i)];
-  const C vkp = FWD ? z : v[ixv(n1, n2, k + 1, j, i)], vkm = v[ixv(n1, n2, k - 1, j, i)];
-  const int kf = k + g.kstart;
   // the conductivities of the six faces around node (k,j,i): the reference reads the
   // lower faces unshifted (Q2, fdfd.c:666,668,670,695,697,699); with aphi_fix all six
   // come from the shifted operator-grid arrays
@@ -301,12 +297,21 @@ __global__ void k_aphi_phi(SweepP<P> s, typename P::C* __restrict__ VV, int t)
   const R s1m = s.aphi_fix ? g.s11[ix1(n1, n2, k, j, i - 1)] : s.s11u[ix1(n1, n2, k, j, i - 1)];
   const R s2m = s.aphi_fix ? g.s22[ix2(n1, n2, k, j - 1, i)] : s.s22u[ix2(n1, n2, k, j - 1, i)];
   const R s3m = s.aphi_fix ? g.s33[ix3(n1, n2, k - 1, j, i)] : s.s33u[ix3(n1, n2, k - 1, j, i)];
-  C t1 = rmul<P>(s1p, cadd<P>(ax[ix1(n1, n2, k, j, i)], cdivs<P>(csub<P>(vip, vp), g.d1s[i], g.r1s[i])));
-  C t2 = rmul<P>(s1m, cadd<P>(ax[ix1(n1, n2, k, j, i - 1)], cdivs<P>(csub<P>(vp, vim), g.d1s[i - 1], g.r1s[i - 1])));
-  C t3 = rmul<P>(s2p, cadd<P>(ay[ix2(n1, n2, k, j, i)], cdivs<P>(csub<P>(vjp, vp), g.d2s[j], g.r2s[j])));
-  C t4 = rmul<P>(s2m, cadd<P>(ay[ix2(n1, n2, k, j - 1, i)], cdivs<P>(csub<P>(vp, vjm), g.d2s[j - 1], g.r2s[j - 1])));
-  C t5 = rmul<P>(s3p, cadd<P>(az[ix3(n1, n2, k, j, i)], cdivs<P>(csub<P>(vkp, vp), g.d3s[k], g.r3s[k])));
-  C t6 = rmul<P>(s3m, cadd<P>(az[ix3(n1, n2, k - 1, j, i)], cdivs<P>(csub<P>(vp, vkm), g.d3s[k - 1], g.r3s[k - 1])));
+  const C a1p = ax[ix1(n1, n2, k, j, i)], a1m = ax[ix1(n1, n2, k, j, i - 1)];
+  const C a2p = ay[ix2(n1, n2, k, j, i)], a2m = ay[ix2(n1, n2, k, j - 1, i)];
+  const C a3p = az[ix3(n1, n2, k, j, i)], a3m = az[ix3(n1, n2, k - 1, j, i)];
+  // all that is older than the sweep's first launch has been asked for: now the hyperplane before
+  cudaGridDependencySynchronize();
+  const C vp = z;  // v(k,j,i) is zeroed before its own update
+  const C vip = FWD ? z : v[ixv(n1, n2, k, j, i + 1)], vim = v[ixv(n1, n2, k, j, i - 1)];
+  const C vjp = FWD ? z : v[ixv(n1, n2, k, j + 1, i)], vjm = v[ixv(n1, n2, k, j - 1, i)];
+  const C vkp = FWD ? z : v[ixv(n1, n2, k + 1, j, i)], vkm = v[ixv(n1, n2, k - 1, j, i)];
+  C t1 = rmul<P>(s1p, cadd<P>(a1p, cdivs<P>(csub<P>(vip, vp), g.d1s[i], g.r1s[i])));
+  C t2 = rmul<P>(s1m, cadd<P>(a1m, cdivs<P>(csub<P>(vp, vim), g.d1s[i - 1], g.r1s[i - 1])));
+  C t3 = rmul<P>(s2p, cadd<P>(a2p, cdivs<P>(csub<P>(vjp, vp), g.d2s[j], g.r2s[j])));
+  C t4 = rmul<P>(s2m, cadd<P>(a2m, cdivs<P>(csub<P>(vp, vjm), g.d2s[j - 1], g.r2s[j - 1])));
+  C t5 = rmul<P>(s3p, cadd<P>(a3p, cdivs<P>(csub<P>(vkp, vp), g.d3s[k], g.r3s[k])));
+  C t6 = rmul<P>(s3m, cadd<P>(a3m, cdivs<P>(csub<P>(vp, vkm), g.d3s[k - 1], g.r3s[k - 1])));
   C aij = cadd<P>(cadd<P>(cdivs<P>(csub<P>(t1, t2), g.d1[i], g.r1[i]), cdivs<P>(csub<P>(t3, t4), g.d2[j], g.r2[j])),
                   cdivs<P>(csub<P>(t5, t6), g.d3[k], g.r3[k]));
   const R one = 1;
@@ -327,7 +332,6 @@ __global__ void k_aphi_phi(SweepP<P> s, typename P::C* __restrict__ VV, int t)
     aii = cmul<P>(aii, f);
   }
   v[ixv(n1, n2, k, j, i)] = cdiv<P>(csub<P>(bv[ixv(n1, n2, k, j, i)], aij), aii);
-  (void)kf;
 }
 
 // E = A + grad v (fdfd.c:796-819), in place on Y
@@ -372,11 +376,12 @@ void launch_aphi_div(const SweepP<P>& s, typename P::C* BV, int nslot, cudaStrea
 template <class P>
 void launch_aphi_phi(const SweepP<P>& s, typename P::C* V, int t, int nslot, cudaStream_t st)
 {
-  // t > 0: forward hyperplane t; t < 0: backward hyperplane -t
-  dim3 blk(32, 4);
-  dim3 grd((s.g.n1 - 1 + 31) / 32, (s.g.n2 - 1 + 3) / 4, nslot);
-  if (t > 0) count_launch(), k_aphi_phi<P, true><<<grd, blk, 0, st>>>(s, V, t);
-  else count_launch(), k_aphi_phi<P, false><<<grd, blk, 0, st>>>(s, V, -t);
+  // t > 0: forward hyperplane t; t < 0: backward hyperplane -t. Each may start before the one
+  // before it ends, and waits for it; the first reads what the kernels before it wrote at once
+  const PlaneLaunch L(s, t, nslot, st);
+  count_launch();
+  if (t > 0) cudaLaunchKernelEx(&L.cfg, k_aphi_phi<P, true>, s, V, t);
+  else cudaLaunchKernelEx(&L.cfg, k_aphi_phi<P, false>, s, V, -t);
 }
 
 template <class P>

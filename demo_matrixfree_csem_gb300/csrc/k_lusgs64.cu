@@ -473,7 +473,8 @@ __global__ void __launch_bounds__(PAIR ? 2 * MAXR : MAXR, PAIR && MAXR <= 128 ? 
 // host-made terms, and the others take no FP64 operation. A node where a quotient is out of range
 // is done again with the / operator. What is left is bound by latency, at some 6 us a hyperplane
 // (84^3 cells: 17 with the divisions; 474 hyperplanes an application, which takes 5.2 ms instead
-// of 10.7, 2.4 instead of 4.4 where three overlap).
+// of 10.7, 2.4 instead of 4.4 where three overlap; and 4.3 and 2.1 with a hyperplane's blocks
+// started, and what does not depend on it loaded, while the one before still runs).
 template <bool FWD>
 __global__ void __launch_bounds__(128) k_aphi_phi64(const __grid_constant__ SweepP<F64> s, C* __restrict__ VV, int t)
 {
@@ -481,6 +482,7 @@ __global__ void __launch_bounds__(128) k_aphi_phi64(const __grid_constant__ Swee
   const GridP<F64>& g = s.g;
   const int n1 = g.n1, n2 = g.n2, n3 = g.n3;
   const int i = 1 + blockIdx.x * 32 + threadIdx.x, j = 1 + blockIdx.y * 4 + threadIdx.y, k = t - i - j;
+  cudaTriggerProgrammaticLaunchCompletion();  // the next hyperplane's blocks may come in and wait
   if (i >= n1 || j >= n2 || k < 1 || k >= n3) return;
   const int sys = s.sys_list ? s.sys_list[slot] : slot;
   C* v = VV + (size_t)slot * s.lv;
@@ -492,27 +494,33 @@ __global__ void __launch_bounds__(128) k_aphi_phi64(const __grid_constant__ Swee
   const double geo = F64::add(F64::add(ro(g.g1 + i), ro(g.g2 + j)), ro(g.g3 + k));
   const C b = ro(s.BV + (size_t)slot * s.lv + q);
   const SysScal<F64> sc = s.scal[sys];
+  // everything but v is older than the sweep's first launch: read it before waiting for the
+  // hyperplane before (which some block of every hyperplane does, so they end in order)
+  const double s1p = ro(g.s11 + ix1(n1, n2, k, j, i)), s1m = ro(s.s11u + ix1(n1, n2, k, j, i - 1));
+  const double s2p = ro(g.s22 + ix2(n1, n2, k, j, i)), s2m = ro(s.s22u + ix2(n1, n2, k, j - 1, i));
+  const double s3p = ro(g.s33 + ix3(n1, n2, k, j, i)), s3m = ro(s.s33u + ix3(n1, n2, k - 1, j, i));
+  const C a1p = ro(ax + ix1(n1, n2, k, j, i)), a1m = ro(ax + ix1(n1, n2, k, j, i - 1));
+  const C a2p = ro(ay + ix2(n1, n2, k, j, i)), a2m = ro(ay + ix2(n1, n2, k, j - 1, i));
+  const C a3p = ro(az + ix3(n1, n2, k, j, i)), a3m = ro(az + ix3(n1, n2, k - 1, j, i));
+  uint32_t bad = 0;
+  const XdDen den = xd_den(-geo, bad);
+  cudaGridDependencySynchronize();
   auto node = [&](auto over_) {
     // sigma (a + (hi - lo) / ds) on a face; v is zero at the node itself
     auto face = [&](double sg, C a, C dv, Sp ds) { return rmul<F64>(sg, cadd<F64>(a, over_(dv, ds))); };
     auto axis = [&](C up, C lo, double sp, double sm, C ap, C am, const Ax64& A) {
       return over_(csub<F64>(face(sp, ap, up, A.s), face(sm, am, csub<F64>(z, lo), A.sm)), A.c);
     };
-    const C x = axis(FWD ? z : v[ix3(n1, n2, k, j, i + 1)], v[q - 1], ro(g.s11 + ix1(n1, n2, k, j, i)),
-                     ro(s.s11u + ix1(n1, n2, k, j, i - 1)), ro(ax + ix1(n1, n2, k, j, i)), ro(ax + ix1(n1, n2, k, j, i - 1)), X);
-    const C y = axis(FWD ? z : v[ix3(n1, n2, k, j + 1, i)], v[qj], ro(g.s22 + ix2(n1, n2, k, j, i)),
-                     ro(s.s22u + ix2(n1, n2, k, j - 1, i)), ro(ay + ix2(n1, n2, k, j, i)), ro(ay + ix2(n1, n2, k, j - 1, i)), Y);
-    const C w = axis(FWD ? z : v[ix3(n1, n2, k + 1, j, i)], v[qk], ro(g.s33 + ix3(n1, n2, k, j, i)),
-                     ro(s.s33u + ix3(n1, n2, k - 1, j, i)), ro(az + ix3(n1, n2, k, j, i)), ro(az + ix3(n1, n2, k - 1, j, i)), Z);
+    const C x = axis(FWD ? z : v[ix3(n1, n2, k, j, i + 1)], v[q - 1], s1p, s1m, a1p, a1m, X);
+    const C y = axis(FWD ? z : v[ix3(n1, n2, k, j + 1, i)], v[qj], s2p, s2m, a2p, a2m, Y);
+    const C w = axis(FWD ? z : v[ix3(n1, n2, k + 1, j, i)], v[qk], s3p, s3m, a3p, a3m, Z);
     return cadd<F64>(cadd<F64>(x, y), w);
   };
-  uint32_t bad = 0;
   C aij = node([&](C a, Sp d) { return over(a, d, bad); });
   C r = z;
   if (!g.fvm) {
-    const XdDen n = xd_den(-geo, bad);
     const C a = csub<F64>(b, aij);
-    r = make_double2(xd_div2(a.x, n.d, n.R, bad), xd_div2(a.y, n.d, n.R, bad));
+    r = make_double2(xd_div2(a.x, den.d, den.R, bad), xd_div2(a.y, den.d, den.R, bad));
   }
   if (bad || g.fvm) {
     if (bad) aij = node([&](C a, Sp d) { return cdivr<F64>(a, d.d); });
@@ -529,10 +537,10 @@ __global__ void __launch_bounds__(128) k_aphi_phi64(const __grid_constant__ Swee
 
 void launch_aphi_phi64(const SweepP<F64>& s, double2* V, int t, int nslot, cudaStream_t st)
 {
-  const dim3 blk(32, 4), grd((s.g.n1 - 1 + 31) / 32, (s.g.n2 - 1 + 3) / 4, nslot);
+  const PlaneLaunch L(s, t, nslot, st);
   count_launch();
-  if (t > 0) k_aphi_phi64<true><<<grd, blk, 0, st>>>(s, V, t);
-  else k_aphi_phi64<false><<<grd, blk, 0, st>>>(s, V, -t);
+  if (t > 0) cudaLaunchKernelEx(&L.cfg, k_aphi_phi64<true>, s, V, t);
+  else cudaLaunchKernelEx(&L.cfg, k_aphi_phi64<false>, s, V, -t);
 }
 
 template <int COMP, bool FWD, bool APHI>
