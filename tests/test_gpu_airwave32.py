@@ -1,4 +1,4 @@
-"""The complex64 airwave's line transforms (csrc/k_airwave32.cu) against the complex128 oracle
+"""The complex64 airwave's line transforms (csrc/k_airlines.cu) against the complex128 oracle
 at each length a side can have, more and fewer rows than a CTA takes, and sizes that stay with two-dimensional transforms (two lengths, other lengths, more
 rows than the uniform grid). Bound 2e-5 of the largest value, that of every complex64 operator
 here; the transforms' own error is about 2^-24 times the 20 roundings of 1024 points."""
