@@ -13,7 +13,8 @@
 // values that no output takes, as do the extra lanes; the first plane's fields above come as
 // the loop's carried values (the airwave's ghosts, fdfd.c:151-172); the last plane of Ex and
 // Ey, which only holds zeros, is written apart; and addresses are 32-bit offsets from the
-// system's vector, advanced by one addition per component and plane.
+// system's component (64-bit where one has more than 2^29 points, 4 GiB), advanced by one addition
+// per component and plane.
 // 200 x 140 x 130 cells, 16 systems: 814 us, 3.5 TB/s of DRAM traffic (1049 us with predicated
 // loads and 64-bit addresses); tiles 4 and 16 rows high 850 and 1070 us. Of about 230
 // instructions a warp and plane 70 are arithmetic; registers (72, for three CTAs of 8 rows
@@ -22,6 +23,7 @@
 #include "csem_cuda.cuh"
 #include "engine.h"
 #include "k_dot_common.cuh"
+#include "offsets32.h"
 
 namespace csem {
 
@@ -29,8 +31,11 @@ namespace {
 
 typedef float2 C;
 
-__device__ __forceinline__ C ld(const char* base, unsigned off) { return __ldg((const C*)(base + off)); }
-__device__ __forceinline__ float ldf(const char* base, unsigned off) { return __ldg((const float*)(base + off)); }
+template <class Off> __device__ __forceinline__ C ld(const char* base, Off off) { return __ldg((const C*)(base + off)); }
+template <class Off> __device__ __forceinline__ float ldf(const char* base, Off off)
+{
+  return __ldg((const float*)(base + off));
+}
 __device__ __forceinline__ C up(C v) { return make_float2(__shfl_up_sync(~0u, v.x, 1), __shfl_up_sync(~0u, v.y, 1)); }
 __device__ __forceinline__ C down(C v) { return make_float2(__shfl_down_sync(~0u, v.x, 1), __shfl_down_sync(~0u, v.y, 1)); }
 // (roundings written out, so that a value is the same whichever code forms it: the bits do
@@ -66,7 +71,7 @@ struct Plane {
 // and writes part[slot][cta] (EPI 2: and part[nslot + slot][cta]), which launch_dot_finish
 // adds up in a fixed order: deterministic, but a different partition of the sum than
 // launch_dot's.
-template <int BY, int EPI>
+template <int BY, int EPI, class Off>
 __global__ void __launch_bounds__(32 * (BY + 1), BY >= 16 ? 1 : (BY >= 8 ? 3 : 5))
     k_fdfd32(GridP<F32> g, const SysScal<F32>* __restrict__ scal, const C* __restrict__ X, C* __restrict__ Y,
              const C* __restrict__ GHX, const C* __restrict__ GHY, int kchunk, int nkc, const int* __restrict__ sys_list,
@@ -87,8 +92,7 @@ __global__ void __launch_bounds__(32 * (BY + 1), BY >= 16 ? 1 : (BY >= 8 ? 3 : 5
   char* const by = (char*)(Y + so + g.lEx);
   char* const bz = (char*)(Y + so + g.lEx + g.lEy);
   const C iwmu = scal[sys].iwmu, iom = scal[sys].iom;
-  const unsigned sX = 8u * (unsigned)(n1 * (n2 + 1)), sY = 8u * (unsigned)((n1 + 1) * n2),
-                 sZ = 8u * (unsigned)((n1 + 1) * (n2 + 1));  // bytes from plane to plane
+  const Off sX = 8 * (Off)n1 * (n2 + 1), sY = 8 * (Off)(n1 + 1) * n2, sZ = 8 * (Off)(n1 + 1) * (n2 + 1);  // bytes from plane to plane
   const char* const s11 = (const char*)(g.s11) + (size_t)ks * (sX / 2);
   const char* const s22 = (const char*)(g.s22) + (size_t)ks * (sY / 2);
   const char* const s33 = (const char*)(g.s33) + (size_t)ks * (sZ / 2);
@@ -97,9 +101,9 @@ __global__ void __launch_bounds__(32 * (BY + 1), BY >= 16 ? 1 : (BY >= 8 ? 3 : 5
   const bool mine = lane >= 1 && lane <= 30 && w >= 1 && i <= n1 && j <= n2;
   const bool outX = mine && i < n1, outY = mine && j < n2, outZ = mine;
   const bool inX = j >= 1 && j <= n2 - 1, inY = i >= 1 && i <= n1 - 1, inZ = inX && inY;
-  unsigned oX = 8u * (unsigned)(ix + n1 * jx) + (unsigned)kb * sX, oY = 8u * (unsigned)(iy + (n1 + 1) * jy) + (unsigned)kb * sY,
-           oZ = 8u * (unsigned)(iy + (n1 + 1) * jx) + (unsigned)kb * sZ;
-  const unsigned upX = jx < n2 ? 8u * n1 : 0u, upZ = jx < n2 ? 8u * (n1 + 1) : 0u;  // to row j + 1
+  Off oX = point_offset<Off>(ix, jx, kb, n1, sX), oY = point_offset<Off>(iy, jy, kb, n1 + 1, sY),
+      oZ = point_offset<Off>(iy, jx, kb, n1 + 1, sZ);
+  const Off upX = jx < n2 ? 8 * (Off)n1 : 0, upZ = jx < n2 ? 8 * (Off)(n1 + 1) : 0;  // to row j + 1
   const float r1s = g.r1s[ix], r1 = g.r1[iy], r2s = g.r2s[jy], r2 = g.r2[jx];
   const float v1s = g.d1s[ix], v1 = g.d1[iy], v2s = g.d2s[jy], v2 = g.d2[jx];
   const C z = make_float2(0.f, 0.f);
@@ -107,7 +111,7 @@ __global__ void __launch_bounds__(32 * (BY + 1), BY >= 16 ? 1 : (BY >= 8 ? 3 : 5
   const char* const eY = EPI ? (const char*)(E + so + g.lEx) : nullptr;
   const char* const eZ = EPI ? (const char*)(E + so + g.lEx + g.lEy) : nullptr;
   DotAcc<F32> dacc1, dacc2;
-  auto put = [&](char* out, const char* e, unsigned o, C y) {
+  auto put = [&](char* out, const char* e, Off o, C y) {
     *(C*)(out + o) = y;
     if constexpr (EPI == 1) {
       dacc1.add(y, ld(e, o));
@@ -117,7 +121,7 @@ __global__ void __launch_bounds__(32 * (BY + 1), BY >= 16 ? 1 : (BY >= 8 ? 3 : 5
     }
   };
 
-  auto load = [&](unsigned x, unsigned y, unsigned zz) {
+  auto load = [&](Off x, Off y, Off zz) {
     Plane p;
     p.ez = ld(Ez, zz);
     p.ezj = ld(Ez, zz + upZ);
@@ -223,15 +227,20 @@ void launch_by(const GridP<F32>& g, const SysScal<F32>* scal, const C* X, C* Y, 
   if (by != 4 && by != 16) by = 8;
   const FdfdShape f = fdfd_shape(g.n1, g.n2, g.n3, nsys, by, ctas_per_sm, FDFD32_TILE);
   dim3 blk(32, by + 1), grd(f.gx, f.gy, nsys * f.nkc);
-  auto go = [&](auto tile) {
+  auto go = [&](auto tile, auto off) {
     constexpr int BY = decltype(tile)::value;
+    typedef decltype(off) Off;
     // of 228 KB; three CTAs use 28 (16 systems' operators on three streams: 1094 -> 921 us each)
-    keep_l1<k_fdfd32<BY, EPI>>(20);
-    count_launch(), k_fdfd32<BY, EPI><<<grd, blk, 0, st>>>(g, scal, X, Y, ghx, ghy, f.kchunk, f.nkc, sys_list, E, part);
+    keep_l1<k_fdfd32<BY, EPI, Off>>(20);
+    count_launch(), k_fdfd32<BY, EPI, Off><<<grd, blk, 0, st>>>(g, scal, X, Y, ghx, ghy, f.kchunk, f.nkc, sys_list, E, part);
   };
-  if (by == 4) go(std::integral_constant<int, 4>());
-  else if (by == 16) go(std::integral_constant<int, 16>());
-  else go(std::integral_constant<int, 8>());
+  auto with = [&](auto off) {
+    if (by == 4) go(std::integral_constant<int, 4>(), off);
+    else if (by == 16) go(std::integral_constant<int, 16>(), off);
+    else go(std::integral_constant<int, 8>(), off);
+  };
+  if (offsets32_reach(g.n1, g.n2, g.n3)) with(0u);
+  else with((size_t)0);
 }
 
 }  // namespace
