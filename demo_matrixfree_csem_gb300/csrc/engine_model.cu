@@ -353,6 +353,14 @@ template <class P> bool Ops<P>::line_fits(int nK) const
          sweep_line_fits(m->n1, m->n2, nK);
 }
 
+template <class P> void Ops<P>::sweep_scratch(long sbs)
+{
+  const size_t b = sizeof(float4) * (size_t)sbs * nmax;
+  if (sb.bytes >= b) return;
+  if (sb.p) moves++;
+  sb.alloc(b);
+}
+
 template <class P> int Ops<P>::split_ctas() const { return split_cap > 0 ? split_cap * sm_count() : 0; }
 
 template <class P>
@@ -500,7 +508,7 @@ void Ops<P>::apply_lusgs(const C* X, C* Y, int nslot, const int* sys_list, const
     if (lines) {
       if (!bounds_zero) launch_line_bounds(s, nslot, st);
       const long sbs = sweep_split_scratch(n1, n2, s.nK);
-      if (sb.bytes < sizeof(float4) * (size_t)sbs * nmax) sb.alloc(sizeof(float4) * (size_t)sbs * nmax);
+      sweep_scratch(sbs);
       float2 *B = sb.as<float2>(), *W = B + (size_t)nslot * sbs;
       const int* groups = g16 && grp->of_slot ? grp->dev : nullptr;
       auto one = [&](int comp, bool fwd) {
@@ -519,7 +527,7 @@ void Ops<P>::apply_lusgs(const C* X, C* Y, int nslot, const int* sys_list, const
     if (split_sweeps && split_overlap && pipelined_sweeps && !tiled_sweeps && all_fit && aux && grp &&
         grp->ns == SPLIT_GROUP && grp->nA > 0 && grp->nA < nslot && grp->ngA > 0 && grp->ngA < grp->n) {
       const long sbs = sweep_split_scratch(n1, n2, s.nK);
-      if (sb.bytes < sizeof(float4) * (size_t)sbs * nmax) sb.alloc(sizeof(float4) * (size_t)sbs * nmax);
+      sweep_scratch(sbs);
       const int nA = grp->nA, nB = nslot - nA, vw = sweep_vw == 1 || sweep_vw == 4 ? sweep_vw : 2;
       SweepP<P> sB = s;
       if (s.sys_list) {
@@ -566,7 +574,7 @@ void Ops<P>::apply_lusgs(const C* X, C* Y, int nslot, const int* sys_list, const
       }
       if (split_sweeps && pipelined_sweeps && sweep_pipelined_fits(comp, n1, n2, s.nK)) {
         const long sbs = sweep_split_scratch(n1, n2, s.nK);
-        if (sb.bytes < sizeof(float4) * (size_t)sbs * nmax) sb.alloc(sizeof(float4) * (size_t)sbs * nmax);
+        sweep_scratch(sbs);
         // groups built as two halves number their slots within each half: here, on one
         // stream, the pass then takes the slots one by one
         const bool g16 = grp && grp->ns == SPLIT_GROUP && grp->n > 0 && grp->nA == 0;
@@ -625,7 +633,7 @@ void Ops<P>::apply_aphi(const C* X, C* Y, int nslot, const int* sys_list, const 
   const long sbs = sweep_split_scratch(n1, n2, n3);
   if constexpr (!P::exact) {
     if (lines) {
-      if (sb.bytes < sizeof(float4) * (size_t)sbs * nmax) sb.alloc(sizeof(float4) * (size_t)sbs * nmax);
+      sweep_scratch(sbs);
       if (!rhs.p) rhs.alloc(sizeof(C) * (size_t)m->lE * nmax);
       launch_line_bounds(s, nslot, st);
     }

@@ -183,6 +183,10 @@ class Ops {
                    bool bounds_zero = false, const SweepGroups* grp = nullptr);
   void apply_aphi(const C* X, C* Y, int nslot, const int* sys_list, const SysScal<P>* sc);
   void zero(C* Y, long n, int nslot, const int* sys_list);
+  // sb for sbs entries a slot. LU-SGS with the air above the model sweeps more planes than A-phi,
+  // so it may move: moves counts that, for those who keep its address (captured graphs)
+  void sweep_scratch(long sbs);
+  unsigned moves = 0;
   void diag_table(const SweepP<P>& s, int nslot);  // complex128: the pipelined sweeps' diagonal table
   int split_ctas() const;  // the split pipelines' grid cap on two streams: split_cap CTAs per SM (0: none)
   ~Ops();

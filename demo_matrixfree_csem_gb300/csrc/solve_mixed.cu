@@ -85,6 +85,16 @@ void MixedBatch::drop_gmres_graphs()
   gm_graphs_.clear();
 }
 
+void MixedBatch::check_graphs()
+{
+  if (seen_moves_ == o32.moves) return;
+  seen_moves_ = o32.moves;
+  drop_gmres_graphs();
+  for (auto& kv : graphs_)
+    if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
+  graphs_.clear();
+}
+
 MixedBatch::~MixedBatch()
 {
   for (auto* m : {&graphs_, &gm_graphs_})
@@ -135,6 +145,7 @@ void MixedBatch::run_captured(Graph& g, bool use_graphs, const std::function<voi
 void MixedBatch::inner_iterations(int nact, const MixedOptions& o)
 {
   const int* dl = list.as<int>();
+  check_graphs();
   run_captured(graphs_[std::make_tuple(nact, o.preco, o.check_every, o.niter, grp_.n * 32 + grp_.ns, grp_.nA, grp_.ngA)],
                o.graphs, [&]() {
     for (int q = 0; q < o.check_every; q++) inner_iteration(nact, dl, o.preco, o.niter);
@@ -684,6 +695,7 @@ void MixedBatch::gmres_inner(const std::vector<int>& g, const std::vector<double
       dim3 grd((unsigned)((n + 255) / 256), (unsigned)na);
       count_launch(), k_gm_update<<<grd, 256, 0, this->st>>>(n, dl, st, ycoef, nsys, GZ(0), N, GD);
     };
+    check_graphs();
     run_captured(gm_graphs_[std::make_tuple(na, m, o.preco, 0, grp_.n * 32 + grp_.ns, grp_.nA, grp_.ngA)], o.graphs,
                  steps);
     CSEM_CUDA_TRY(cudaGetLastError());
