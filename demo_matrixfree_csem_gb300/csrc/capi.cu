@@ -48,21 +48,27 @@ struct csem_ctx {
 // the context's kernel-schedule options on one operator set
 template <class P> static void configure(const csem_ctx* c, Ops<P>& o)
 {
-  o.pipelined_sweeps = c->lusgs_pipelined;
-  o.sweep_vw = c->lusgs_vw;
-  o.sweep_lines = c->lusgs_lines;
-  o.sweep_systems = c->lusgs_systems;
-  o.split_sweeps = c->lusgs_split != 0;
-  o.line_sweeps = c->lusgs_split == 2;
-  o.split_overlap = c->lusgs_overlap;
-  o.fused_dots = c->fused_dots;
-  o.split_cap = c->lusgs_cap;
-  o.stencil_by = c->stencil_by;
-  o.stencil_ctas = c->stencil_ctas;
-  o.tiled_sweeps = c->lusgs_tiled;
-  o.aphi_fix = c->aphi_fix;
-  o.tile_rows = c->tile_rows;
-  o.tile_vw = c->tile_vw;
+  bool changed = false;
+  auto set = [&](auto& option, auto value) {
+    changed = changed || option != value;
+    option = value;
+  };
+  set(o.pipelined_sweeps, c->lusgs_pipelined);
+  set(o.sweep_vw, c->lusgs_vw);
+  set(o.sweep_lines, c->lusgs_lines);
+  set(o.sweep_systems, c->lusgs_systems);
+  set(o.split_sweeps, c->lusgs_split != 0);
+  set(o.line_sweeps, c->lusgs_split == 2);
+  set(o.split_overlap, c->lusgs_overlap);
+  set(o.fused_dots, c->fused_dots);
+  set(o.split_cap, c->lusgs_cap);
+  set(o.stencil_by, c->stencil_by);
+  set(o.stencil_ctas, c->stencil_ctas);
+  set(o.tiled_sweeps, c->lusgs_tiled);
+  set(o.aphi_fix, c->aphi_fix);
+  set(o.tile_rows, c->tile_rows);
+  set(o.tile_vw, c->tile_vw);
+  if (changed) o.epoch++;
 }
 
 #define API_BEGIN try {

@@ -357,7 +357,7 @@ template <class P> void Ops<P>::sweep_scratch(long sbs)
 {
   const size_t b = sizeof(float4) * (size_t)sbs * nmax;
   if (sb.bytes >= b) return;
-  if (sb.p) moves++;
+  if (sb.p) epoch++;
   sb.alloc(b);
 }
 

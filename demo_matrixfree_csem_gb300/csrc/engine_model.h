@@ -184,9 +184,11 @@ class Ops {
   void apply_aphi(const C* X, C* Y, int nslot, const int* sys_list, const SysScal<P>* sc);
   void zero(C* Y, long n, int nslot, const int* sys_list);
   // sb for sbs entries a slot. LU-SGS with the air above the model sweeps more planes than A-phi,
-  // so it may move: moves counts that, for those who keep its address (captured graphs)
+  // so it may move
   void sweep_scratch(long sbs);
-  unsigned moves = 0;
+  // counts what makes launches captured earlier other than those of now: sb moved, or one of the
+  // options above changed
+  unsigned epoch = 0;
   void diag_table(const SweepP<P>& s, int nslot);  // complex128: the pipelined sweeps' diagonal table
   int split_ctas() const;  // the split pipelines' grid cap on two streams: split_cap CTAs per SM (0: none)
   ~Ops();

@@ -87,8 +87,8 @@ void MixedBatch::drop_gmres_graphs()
 
 void MixedBatch::check_graphs()
 {
-  if (seen_moves_ == o32.moves) return;
-  seen_moves_ = o32.moves;
+  if (epoch_ == o32.epoch) return;
+  epoch_ = o32.epoch;
   drop_gmres_graphs();
   for (auto& kv : graphs_)
     if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
@@ -314,6 +314,11 @@ int MixedBatch::autotune_lusgs(const std::vector<int>& running)
     return ms;
   };
   const bool saved = o32.pipelined_sweeps, saved_tiled = o32.tiled_sweeps;
+  auto chosen = [&]() {
+    return std::make_tuple(o32.split_sweeps, o32.line_sweeps, o32.sweep_systems, o32.sweep_vw, o32.sweep_lines,
+                           o32.stencil_by, o32.stencil_ctas);
+  };
+  const auto before = chosen();
   o32.pipelined_sweeps = true;
   o32.tiled_sweeps = false;
   float best_ms = 1e30f;
@@ -364,6 +369,7 @@ int MixedBatch::autotune_lusgs(const std::vector<int>& running)
     }
   o32.stencil_by = best_by;
   o32.stencil_ctas = best_ctas;
+  if (chosen() != before) o32.epoch++;
   tuned_lines = best_lines;
   tuned_systems = best_ns;
   tuned_split = best_split;

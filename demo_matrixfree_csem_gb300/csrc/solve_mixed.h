@@ -76,9 +76,9 @@ class MixedBatch {
   // graph from the second time on (never while per-operator profiling records events)
   void run_captured(Graph& g, bool use_graphs, const std::function<void()>& body);
   void drop_gmres_graphs();  // before the GMRES buffers move
-  // drops every graph if o32's scratch has moved since the last call; before a graph is looked up
+  // drops every graph if o32's epoch is not the last call's; before a graph is looked up
   void check_graphs();
-  unsigned seen_moves_ = 0;
+  unsigned epoch_ = 0;
   void start_inner(const std::vector<int>& g, const std::vector<double>& tol_inner);
   // the active systems into list and, for grouped complex64 sweeps (o32.sweep_systems >
   // 1), their same-frequency groups into grp_
