@@ -203,8 +203,7 @@ int csem_ctx_set_option(csem_ctx* c, const char* name, int value)
     if (value != 1 && value != 2 && value != 4) return csem_set_error(CSEM_EINVAL, "lusgs_systems must be 1, 2 or 4");
     c->lusgs_systems = value;
   } else if (!strcmp(name, "lusgs_split")) {
-    if (value < 0 || value > 2) return csem_set_error(CSEM_EINVAL, "lusgs_split must be 0, 1 or 2");
-    c->lusgs_split = value;
+    c->lusgs_split = value == 0 || value == 1 ? value : 2;  // (once a switch: any value but 0 was on)
   } else if (!strcmp(name, "quick_residual")) {
     c->quick_residual = value != 0;
   } else if (!strcmp(name, "fused_dots")) {

@@ -247,8 +247,8 @@ void *csem_ctx_stream(csem_ctx *c);
  *                     and, once for the systems of a frequency, w = iwmu/aii, and a chain
  *                     with a warp per line; 1: the pass and a row pipeline with a thread
  *                     per row, in the chain's place also where a grid is too large for it;
- *                     0: the one-pass pipelined sweeps. Same values to rounding. 2
- *                     also runs A-phi's edge sweeps so, else by diagonals;
+ *                     0: the one-pass pipelined sweeps; other values as 2. Same values to
+ *                     rounding. 2 also runs A-phi's edge sweeps so, else by diagonals;
  *   "quick_residual"  1 (default): the batched mixed-precision solve forms its complex128
  *                     residuals r = b - A x with a complex128 stencil that multiplies by
  *                     reciprocal spacings and lets the compiler contract multiply-adds
