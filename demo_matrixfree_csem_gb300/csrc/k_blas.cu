@@ -8,6 +8,7 @@
 // summed per thread with a compensated (TwoSum) float pair, so the per-thread partials
 // carry ~48 significant bits; partials are combined in FP64.
 #include <cooperative_groups.h>
+#include <type_traits>
 #include "csem_cuda.cuh"
 #include "engine.h"
 #include "solver_state.h"
@@ -92,6 +93,23 @@ __device__ __forceinline__ void block_sum_to(double2 v1, double2 v2, double2* ds
   }
 }
 
+// a thread's sum of a*conj(b) over beg, beg + DOT_THREADS, .. below end, Acc's way
+template <class Acc, class C>
+__device__ __forceinline__ double2 thread_sum(const C* __restrict__ a, const C* __restrict__ b, long beg, long end)
+{
+  Acc d;
+#pragma unroll 4
+  for (long q = beg; q < end; q += DOT_THREADS) d.add(a[q], b[q]);
+  if constexpr (std::is_same<Acc, NormAcc64>::value) {
+    if (d.again()) {
+      NormAcc64::General g;
+      for (long q = beg; q < end; q += DOT_THREADS) g.add(a[q], b[q]);
+      return g.value();
+    }
+  }
+  return d.value();
+}
+
 // partial[slot][blk] = sum over the block's chunk of a*conj(b), Acc's way
 template <class P, class Acc>
 __global__ void __launch_bounds__(DOT_THREADS)
@@ -104,10 +122,7 @@ k_dot_partial(const typename P::C* __restrict__ A, const typename P::C* __restri
   const typename P::C* b = B + (size_t)sys * stride;
   const long chunk = (n + nblk - 1) / nblk;
   const long beg = (long)blockIdx.x * chunk, end = min(n, beg + chunk);
-  Acc d;
-#pragma unroll 4
-  for (long q = beg + threadIdx.x; q < end; q += DOT_THREADS) d.add(a[q], b[q]);
-  block_sum_to(d.value(), partial + (size_t)slot * nblk + blockIdx.x);
+  block_sum_to(thread_sum<Acc>(a, b, beg + threadIdx.x, end), partial + (size_t)slot * nblk + blockIdx.x);
 }
 
 // The whole dot product of a short vector (nblk <= DOT_CLUSTER) in one launch. The warps of
@@ -130,10 +145,7 @@ k_dot_short(const typename P::C* __restrict__ A, const typename P::C* __restrict
   const int warp = blockIdx.x * nblk + w, blk = warp / WARPS;  // of all warps; its block
   const long chunk = (n + nblk - 1) / nblk;
   const long beg = (long)blk * chunk, end = min(n, beg + chunk);
-  Acc d;
-#pragma unroll 4
-  for (long q = beg + 32 * (warp % WARPS) + lane; q < end; q += DOT_THREADS) d.add(a[q], b[q]);
-  double2 v = warp_sum(d.value());
+  double2 v = warp_sum(thread_sum<Acc>(a, b, beg + 32 * (warp % WARPS) + lane, end));
   if (lane == 0) sums[w] = v;
   cg::cluster_group cluster = cg::this_cluster();
   cluster.sync();

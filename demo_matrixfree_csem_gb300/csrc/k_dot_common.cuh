@@ -70,14 +70,17 @@ template <> struct DotAcc<F32> {
 };
 
 // <a, a> in complex128: the real part in DotAcc<F64>'s operations and order (4 instead of 8, which
-// bind it: the imaginary part is a sum of exact zeros)
+// bind it: the imaginary part is a sum of exact zeros). Only where the sum is infinite or NaN can a
+// product of the two parts be: there the values are summed again by DotAcc<F64>
 struct NormAcc64 {
+  typedef DotAcc<F64> General;
   double acc = 0;
+  __device__ __forceinline__ bool again() const { return !isfinite(acc); }
   __device__ __forceinline__ void add(double2 a, double2)
   {
     acc = __dadd_rn(acc, __dadd_rn(__dmul_rn(a.x, a.x), __dmul_rn(a.y, a.y)));
   }
-  __device__ __forceinline__ double2 value() const { return make_double2(acc, isfinite(acc) ? 0. : acc - acc); }
+  __device__ __forceinline__ double2 value() const { return make_double2(acc, 0.); }
 };
 
 template <> struct DotAcc<F64Q> : DotAcc<F64> {};  // the complex128 accumulation
