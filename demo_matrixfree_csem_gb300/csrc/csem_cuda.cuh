@@ -108,6 +108,8 @@ template <class P> struct GridP {
   // is out of its range) and (1/d*s[n] + 1/d*s[n-1]) / d*[n] for n >= 1
   const uint64_t *q1, *q2, *q3, *q1s, *q2s, *q3s;
   const R *g1, *g2, *g3;
+  // complex64 only: (r*s[n] + r*s[n-1]) r*[n] for n >= 1, as the sum of two floats
+  const float2 *gg1, *gg2, *gg3;
 };
 
 // the same grid seen by another precision with the same real type (F64 -> F64Q)
@@ -123,6 +125,7 @@ template <class Q, class P> inline GridP<Q> grid_as(const GridP<P>& g)
   q.s11 = g.s11; q.s22 = g.s22; q.s33 = g.s33;
   q.q1 = g.q1; q.q2 = g.q2; q.q3 = g.q3; q.q1s = g.q1s; q.q2s = g.q2s; q.q3s = g.q3s;
   q.g1 = g.g1; q.g2 = g.g2; q.g3 = g.g3;
+  q.gg1 = g.gg1; q.gg2 = g.gg2; q.gg3 = g.gg3;
   return q;
 }
 

@@ -49,18 +49,27 @@ Model::Model(const csem_grid* gp, int airbc_, int fvm_)
   lv = (long)(n1 + 1) * (n2 + 1) * (n3 + 1);
   rho_water = G.rho_water;
 
-  // 1-D spacings and their reciprocals: 12 arrays, each padded to a common length
+  // 1-D spacings and their reciprocals: 12 arrays, each padded to a common length; complex64 has
+  // 3 more of pairs, the geometric part of the line sweeps' diagonal per axis
   const int L = std::max(n1, std::max(n2, n3f)) + 1;
   const double* src[6] = {G.d1, G.d2, G.d3, G.d1s, G.d2s, G.d3s};
   const int len[6] = {n1 + 1, n2 + 1, n3f + 1, n1 + 1, n2 + 1, n3f + 1};
   std::vector<double> h64((size_t)12 * L, 0.0);
-  std::vector<float> h32((size_t)12 * L, 0.f);
+  std::vector<float> h32((size_t)18 * L, 0.f);
   for (int a = 0; a < 6; a++)
     for (int q = 0; q < len[a]; q++) {
       h64[(size_t)a * L + q] = src[a][q];
       h64[(size_t)(a + 6) * L + q] = 1.0 / src[a][q];
       h32[(size_t)a * L + q] = (float)src[a][q];
       h32[(size_t)(a + 6) * L + q] = (float)(1.0 / src[a][q]);
+    }
+  for (int a = 0; a < 3; a++)
+    for (int q = 1; q < len[a]; q++) {
+      const float *r = &h32[(size_t)(a + 6) * L], *rs = &h32[(size_t)(a + 9) * L];
+      const double g = ((double)rs[q] + (double)rs[q - 1]) * r[q];
+      float* out = &h32[(size_t)(12 + 2 * a) * L + 2 * q];
+      out[0] = (float)g;
+      out[1] = (float)(g - out[0]);
     }
   upload(d64, h64);
   upload(d32, h32);
@@ -108,6 +117,8 @@ Model::Model(const csem_grid* gp, int airbc_, int fvm_)
   memset(&g32, 0, sizeof(g32));
   fill(g64, d64.as<double>(), s64.as<double>());
   fill(g32, d32.as<float>(), s32.as<float>());
+  const float2* pairs = (const float2*)(d32.as<float>() + 12 * L);
+  g32.gg1 = pairs; g32.gg2 = pairs + L; g32.gg3 = pairs + 2 * L;
   const uint64_t* qb = q64.as<uint64_t>();
   if (q_ok) {
     g64.q1 = qb; g64.q2 = qb + L; g64.q3 = qb + 2 * L;
@@ -221,6 +232,7 @@ template <class P> GridP<P> Model::grid_shifted() const
     g.q3s += ks;
   }
   if (g.g3) g.g3 += ks;
+  if (g.gg3) g.gg3 += ks;
   g.s11 += (long)ks * n1 * (n2 + 1);
   g.s22 += (long)ks * (n1 + 1) * n2;
   g.s33 += (long)ks * (n1 + 1) * (n2 + 1);

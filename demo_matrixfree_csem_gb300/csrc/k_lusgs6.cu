@@ -122,6 +122,63 @@ __device__ __forceinline__ long plane(const SweepP<F32>& s, int c, int k, bool u
   return (up ? g.lEx + g.lEy : s.capEx + s.capEy) + kk * (g.n1 + 1) * (g.n2 + 1);
 }
 
+// 1 / (a + i low) as v + c, good to some 2^-40: scaled, so that no square leaves the range, and a step
+// of Newton's iteration from the residual, whose products are formed exactly
+struct Recip {
+  C v, c;
+};
+__device__ __forceinline__ float rcp_approx(float a)
+{
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ Recip recip(C a, float low)
+{
+  const float rm = rcp_approx(fmaxf(fabsf(a.x), fabsf(a.y)));
+  const float xs = a.x * rm, ys = a.y * rm, q = rm * rcp_approx(__fmaf_rn(xs, xs, ys * ys));
+  const float x = xs * q, y = -ys * q;
+  const float h = __fmul_rn(a.x, x), k = -__fmul_rn(a.y, y), m = __fmul_rn(a.y, x);  // h + k is 1, nearly
+  const float hl = __fmaf_rn(a.x, x, -h), kl = -__fmaf_rn(a.y, y, k), ml = __fmaf_rn(a.y, x, -m);
+  const float er = __fsub_rn(__fsub_rn(__fsub_rn(1.f, fmaxf(h, k)), fminf(h, k)), __fsub_rn(__fadd_rn(hl, kl), low * y));
+  const float ei = -__fadd_rn(__fmaf_rn(a.x, y, m), __fmaf_rn(low, x, ml));
+  Recip r;
+  r.v = make_float2(x, y);
+  r.c = make_float2(__fmaf_rn(x, er, -__fmul_rn(y, ei)), __fmaf_rn(x, ei, __fmul_rn(y, er)));
+  return r;
+}
+// What a point and a frequency share: w = iwmu/aii with aii = (ga + gb) iwmu - sg, and 1/aii (with
+// fvm 1/(aii vol iom)), both to the last place of aii from the rounded reciprocal spacings: their
+// errors are the same all along a line, and add up. Of 41 A-phi models the output's error is
+// 0.996 times that of the sweeps by diagonals, which divide (1.025, and up to 1.7, with 1/aii and w
+// of some three places' error), of 16 LU-SGS models 0.60 times that of the row pipelines
+struct Coef {
+  C inv, w;
+};
+__device__ __forceinline__ Coef coef(const SysScal<F32>& sc, int fvm, float2 ga, float2 gb, float sg, float vol)
+{
+  const float g = __fadd_rn(ga.x, gb.x), t = __fsub_rn(g, ga.x);
+  const float gl = __fadd_rn(__fadd_rn(__fsub_rn(ga.x, __fsub_rn(g, t)), __fsub_rn(gb.x, t)), __fadd_rn(ga.y, gb.y));
+  const C iw = sc.iwmu;
+  const float y = __fmul_rn(g, iw.y), yl = __fmaf_rn(gl, iw.y, __fmaf_rn(g, iw.y, -y));
+  const Recip r = recip(make_float2(__fmaf_rn(g, iw.x, -sg), y), yl);
+  Coef c;
+  c.inv = make_float2(__fadd_rn(r.v.x, r.c.x), __fadd_rn(r.v.y, r.c.y));
+  c.w.x = __fmaf_rn(iw.x, r.v.x, __fmaf_rn(-iw.y, r.v.y, __fmaf_rn(iw.x, r.c.x, -__fmul_rn(iw.y, r.c.y))));
+  c.w.y = __fmaf_rn(iw.y, r.v.x, __fmaf_rn(iw.x, r.v.y, __fmaf_rn(iw.y, r.c.x, __fmul_rn(iw.x, r.c.y))));
+  if (fvm) {
+    const Recip f = recip(make_float2(vol * sc.iom.x, vol * sc.iom.y), 0.f);
+    c.inv = mul32(c.inv, make_float2(__fadd_rn(f.v.x, f.c.x), __fadd_rn(f.v.y, f.c.y)));
+  }
+  return c;
+}
+// B = b/aii + w kc (with fvm b/(aii vol iom)), kc = known - cross
+__device__ __forceinline__ C form_B(const Coef& c, C b, C kc)
+{
+  return make_float2(__fmaf_rn(b.x, c.inv.x, __fmaf_rn(-b.y, c.inv.y, __fmaf_rn(c.w.x, kc.x, -__fmul_rn(c.w.y, kc.y)))),
+                     __fmaf_rn(b.x, c.inv.y, __fmaf_rn(b.y, c.inv.x, __fmaf_rn(c.w.x, kc.y, __fmul_rn(c.w.y, kc.x)))));
+}
+
 constexpr int PASS_WARPS = 2;
 // Percent of an SM's 228 KB that the passes leave for shared memory (Ex's uses 34 KB). With the
 // chains' setting (all of it) the passes' loads miss L1: 16 systems 4.81 -> 6.38 ms an
@@ -150,7 +207,8 @@ __global__ void __launch_bounds__(32 * PASS_WARPS, 16)
   const bool on = p < M, pair = j0 + 1 < n2;
   // Ey: row axis Z (k), line axis Y (j); Ez: row axis Y (j), line axis Z (k)
   const Ax<F32> X = axis<F32>(g.d1, g.d1s, g.r1, g.r1s, i);
-  Coef32 cf[2];
+  const float2 gx = ro(g.gg1 + i);
+  Coef cf[2];
   float rr[2], lrs[2], kr[2];  // the row's 1/d, the line's 1/ds, the coupling to the row below
   size_t e[2];
 #pragma unroll
@@ -158,10 +216,10 @@ __global__ void __launch_bounds__(32 * PASS_WARPS, 16)
     const int j = min(j0 + a, n2 - 1);
     const Ax<F32> Rw = COMP == 1 ? axis<F32>(g.d3, g.d3s, g.r3, g.r3s, k) : axis<F32>(g.d2, g.d2s, g.r2, g.r2s, j);
     const Ax<F32> LA = COMP == 1 ? axis_at<F32>(g.d2, g.d2s, g.r2, g.r2s, j) : axis_at<F32>(g.d3, g.d3s, g.r3, g.r3s, k);
-    const float gg = (X.rs + X.rsm) * X.r + (Rw.rs + Rw.rsm) * Rw.r;  // geo(Z, X) / geo(X, Y)
+    const float2 gr = COMP == 1 ? ro(g.gg3 + k) : ro(g.gg2 + j);  // the row axis' part of aii
     const float ydd = COMP == 1 ? LA.d : Rw.d, zdd = COMP == 1 ? Rw.d : LA.d;
     const float sg = ro(COMP == 1 ? g.s22 + ix2(n1, n2, k, j, i) : g.s33 + ix3(n1, n2, k, j, i));
-    cf[a] = lin_coef(sc, g.fvm, gg, sg, X.ds * ydd * zdd);
+    cf[a] = coef(sc, g.fvm, gx, gr, sg, X.ds * ydd * zdd);
     rr[a] = Rw.r;
     lrs[a] = -LA.rs;
     kr[a] = Rw.r * Rw.rsm;
@@ -247,7 +305,7 @@ __global__ void __launch_bounds__(32 * PASS_WARPS, 16)
       }
       C kc = scl32(lrs[a], acc);
       if (!FWD) kc = make_float2(kc.x + (km * v.o[a].x + kr[a] * v.lo[a].x), kc.y + (km * v.o[a].y + kr[a] * v.lo[a].y));
-      const C B = lin_B(cf[a], g.fvm, v.b[a], kc);
+      const C B = form_B(cf[a], v.b[a], kc);
       if (on && (a == 0 || pair)) out[e[a]] = B;
     }
   };
@@ -274,15 +332,15 @@ __global__ void __launch_bounds__(256, 3) k_line_pass_ex(SweepP<F32> s, float2* 
   const bool upA = k >= s.vshift, upB = k - 1 >= s.vshift;
   const Ax<F32> Z = axis<F32>(g.d3, g.d3s, g.r3, g.r3s, k);
   const float xrs = ro(g.r1s + i), xds = ro(g.d1s + i), kz = Z.r * Z.rsm;
-  Coef32 cf[2];
+  const float2 gz = ro(g.gg3 + k);
+  Coef cf[2];
   float yr[2], kj[2];
   unsigned ox[2], oy[2], oz[2], ozm[2], oxm[2];
 #pragma unroll
   for (int a = 0; a < 2; a++) {
     const int st = 16 * blockIdx.y + ty + 8 * a, j = FWD ? min(1 + st, M) : max(M - st, 1);  // (past the last position: it again)
     const Ax<F32> Y = axis<F32>(g.d2, g.d2s, g.r2, g.r2s, j);
-    const float gg = (Y.rs + Y.rsm) * Y.r + (Z.rs + Z.rsm) * Z.r;  // geo(Y, Z)
-    cf[a] = lin_coef(sc, g.fvm, gg, ro(g.s11 + ix1(n1, n2, k, j, i)), xds * Y.d * Z.d);
+    cf[a] = coef(sc, g.fvm, ro(g.gg2 + j), gz, ro(g.s11 + ix1(n1, n2, k, j, i)), xds * Y.d * Z.d);
     yr[a] = Y.r;
     kj[a] = Y.r * Y.rsm;
     ox[a] = 8u * (unsigned)(plane(s, 0, k, upA) + (long)j * n1 + i);
@@ -332,7 +390,7 @@ __global__ void __launch_bounds__(256, 3) k_line_pass_ex(SweepP<F32> s, float2* 
         const C cross = scl32(xrs, make_float2(yr[a] * dy.x + Z.r * dz.x, yr[a] * dy.y + Z.r * dz.y));
         kc = sub32(make_float2(kj[a] * v[a].ej.x + kz * v[a].ek.x, kj[a] * v[a].ej.y + kz * v[a].ek.y), cross);
       }
-      tile[tx][ty + 8 * a] = lin_B(cf[a], g.fvm, v[a].b, kc);
+      tile[tx][ty + 8 * a] = form_B(cf[a], v[a].b, kc);
     }
     if (q + 1 < mem.n) load(q + 1);  // in flight while this system's tile turns
     turn(tile, SB + (size_t)mem.slot_of(q) * sbs);
@@ -382,12 +440,14 @@ __global__ void __launch_bounds__(256) k_aphi_rhs(SweepP<F32> s, C* T)
     const long n = ix3(n1, n2, k, j, i);
     const C hi = ro(v + n + (c == 0 ? 1 : (c == 1 ? L1 : (long)L1 * (n2 + 1)))), lo = ro(v + n);
     const float f = (c == 0 ? ro(g.s11 + r) * ro(g.r1s + i) : (c == 1 ? ro(g.s22 + r) * ro(g.r2s + j) : ro(g.s33 + r) * ro(g.r3s + k)));
-    C e = make_float2(f * (hi.x - lo.x), f * (hi.y - lo.y));
+    const C d = sub32(hi, lo);
     if (g.fvm) {
       const SysScal<F32> sc = s.scal[sys];
-      e = mul32(e, scl32(ro(g.d1s + i) * ro(g.d2 + j) * ro(g.d3 + k), sc.iom));
+      const C e = mul32(scl32(f, d), scl32(ro(g.d1s + i) * ro(g.d2 + j) * ro(g.d3 + k), sc.iom));
+      t = make_float2(t.x + e.x, t.y + e.y);
+    } else {
+      t = make_float2(__fmaf_rn(f, d.x, t.x), __fmaf_rn(f, d.y, t.y));
     }
-    t = make_float2(t.x + e.x, t.y + e.y);
   }
   T[(size_t)sys * g.lE + q] = t;
 }
