@@ -269,9 +269,13 @@ static double batch_bytes(const Model* m, int precision, int preco, int nsys)
   if (precision == 32) {
     // x, b, r, w in complex128; 9 complex64 Krylov vectors; per-system scalars; the split
     // sweeps' (B, w) of the largest component on the sweep grid, and A-phi's right-hand side
-    const double split = preco == PRE_LUSGS
-                             ? 16.0 * (double)sweep_split_scratch(m->n1, m->n2, m->airbc ? m->n3f : m->n3)
-                             : (preco == PRE_APHI ? 16.0 * (double)sweep_split_scratch(m->n1, m->n2, m->n3) + 8.0 * lE : 0.0);
+    const int nK = preco == PRE_LUSGS && m->airbc ? m->n3f : m->n3;
+    const bool lines = sweep_line_fits(m->n1, m->n2, nK);
+    double split = 0;
+    if (preco == PRE_LUSGS)
+      split = 16.0 * std::max(sweep_split_scratch(m->n1, m->n2, nK), lines ? sweep_line_scratch(m->n1, m->n2, nK) : 0);
+    else if (preco == PRE_APHI && lines)
+      split = 16.0 * sweep_line_scratch(m->n1, m->n2, nK) + 8.0 * lE;
     return nsys * (4.0 * 16 * lE + 9.0 * 8 * lE + ops(16) + ops(8) + split + 4096.0);
   }
   // the complex128 solver runs one system at a time: 7 BiCGStab vectors or GMRES(m) bases

@@ -145,7 +145,7 @@ void launch_split_prep(const SweepP<F32>& s, int comp, bool fwd, int nslot, floa
 void launch_split_sweep(const SweepP<F32>& s, int comp, bool fwd, int nslot, const float4* SB, long sbs, int vw,
                         int max_ctas, cudaStream_t st);
 // complex64 sweeps as a pass over the points and a chain with a warp per line (k_lusgs6.cu):
-// the pass stores B per slot and w per group (SB, SW: sbs float2, sweep_split_scratch, per
+// the pass stores B per slot and w per group (SB, SW: sbs float2, sweep_line_scratch, per
 // slot and per group), the chain reads them. groups: ngroups x SPLIT_GROUP slots of one
 // frequency each (null: each slot a group of its own), group_of[slot] a slot's group (null:
 // the slot)
@@ -160,6 +160,7 @@ void launch_sweep_line(const SweepP<F32>& s, int comp, bool fwd, int nslot, cons
 bool sweep_line_fits(int n1, int n2, int nK);  // the rows' tables and edge columns fit shared memory
 int sm_count();  // multiprocessors of the current device
 long sweep_split_scratch(int n1, int n2, int nK);  // largest component on the sweep grid
+long sweep_line_scratch(int n1, int n2, int nK);   // the same as the line sweeps store it
 template <class P>
 void launch_sweep(const SweepP<P>& s, int comp, bool fwd, bool aphi, int t, int nslot, cudaStream_t st);
 int sweep_diagonals(int comp, int n1, int n2, int nK);  // number of diagonals t (2..)

@@ -373,6 +373,23 @@ template <class P> void Ops<P>::sweep_scratch(long sbs)
   sb.alloc(b);
 }
 
+template <class P> bool Ops<P>::line_scratch(long sbs, bool aphi)
+{
+  if (aphi && no_room_aphi) return false;
+  const size_t had = sb.bytes;
+  try {
+    sweep_scratch(sbs);
+    if (aphi && !rhs.p) rhs.alloc(sizeof(C) * (size_t)m->lE * nmax);
+    return true;
+  } catch (const CudaError& e) {
+    if (e.err != cudaErrorMemoryAllocation) throw;
+    (void)cudaGetLastError();  // (not the next launch's)
+    if (sb.bytes != had) sb.free_();
+    (aphi ? no_room_aphi : no_room) = true;
+    return false;
+  }
+}
+
 template <class P> int Ops<P>::split_ctas() const { return split_cap > 0 ? split_cap * sm_count() : 0; }
 
 template <class P>
@@ -479,13 +496,23 @@ int build_sweep_groups_halves(int nslot, const double* iom_of_slot, int ns, int 
 }
 
 template <class P>
-void Ops<P>::diag_table(const SweepP<P>& s, int nslot)
+bool Ops<P>::diag_table(const SweepP<P>& s, int nslot)
 {
   if constexpr (P::exact) {
+    if (!pipelined_sweeps) return false;
     const size_t b = sweep64_table_bytes(m->n1, m->n2, s.nK) * nmax;
-    if (tab.bytes < b) tab.alloc(b);
+    if (tab.bytes < b) {
+      try {
+        tab.alloc(b);
+      } catch (const CudaError& e) {
+        if (e.err != cudaErrorMemoryAllocation) throw;
+        (void)cudaGetLastError();
+        return false;
+      }
+    }
     launch_sweep64_table(s, nslot, tab.p, st);
   }
+  return pipelined_sweeps;
 }
 
 template <class P>
@@ -509,7 +536,8 @@ void Ops<P>::apply_lusgs(const C* X, C* Y, int nslot, const int* sys_list, const
     s.capEy = (long)nb * (n1 + 1) * n2;
     s.capE = s.capEx + s.capEy + (long)nb * (n1 + 1) * (n2 + 1);
   }
-  const bool lines = line_fits();
+  const long lbs = sweep_line_scratch(n1, n2, s.nK);
+  const bool lines = line_fits() && line_scratch(lbs, false);
   if (!bounds_zero && !lines) {
     if (s.CAP) CSEM_CUDA_TRY(cudaMemsetAsync(cap.p, 0, sizeof(C) * (size_t)s.capE * nslot, st));
     zero(Y, m->lE, nslot, sys_list);
@@ -519,13 +547,11 @@ void Ops<P>::apply_lusgs(const C* X, C* Y, int nslot, const int* sys_list, const
     const bool g16 = grp && grp->ns == SPLIT_GROUP && grp->n > 0 && grp->nA == 0;
     if (lines) {
       if (!bounds_zero) launch_line_bounds(s, nslot, st);
-      const long sbs = sweep_split_scratch(n1, n2, s.nK);
-      sweep_scratch(sbs);
-      float2 *B = sb.as<float2>(), *W = B + (size_t)nslot * sbs;
+      float2 *B = sb.as<float2>(), *W = B + (size_t)nslot * lbs;
       const int* groups = g16 && grp->of_slot ? grp->dev : nullptr;
       auto one = [&](int comp, bool fwd) {
-        launch_line_pass(s, comp, fwd, nslot, B, W, sbs, groups, groups ? grp->n : 0, st);
-        launch_sweep_line(s, comp, fwd, nslot, B, W, sbs, groups ? grp->of_slot : nullptr, st);
+        launch_line_pass(s, comp, fwd, nslot, B, W, lbs, groups, groups ? grp->n : 0, st);
+        launch_sweep_line(s, comp, fwd, nslot, B, W, lbs, groups ? grp->of_slot : nullptr, st);
       };
       for (int comp = 0; comp < 3; comp++) one(comp, true);
       for (int comp = 2; comp >= 0; comp--) one(comp, false);
@@ -573,9 +599,7 @@ void Ops<P>::apply_lusgs(const C* X, C* Y, int nslot, const int* sys_list, const
       return;
     }
   }
-  if constexpr (P::exact) {
-    if (pipelined_sweeps) diag_table(s, nslot);
-  }
+  const bool pipelined = diag_table(s, nslot);
   // both schedules visit the points of a sweep in an order that respects every
   // dependency of the lexicographic sweep, so they may be mixed sweep by sweep
   auto sweep = [&](int comp, bool fwd) {
@@ -600,7 +624,7 @@ void Ops<P>::apply_lusgs(const C* X, C* Y, int nslot, const int* sys_list, const
         return;
       }
     }
-    if (pipelined_sweeps && sweep_pipelined_fits(comp, n1, n2, s.nK)) {
+    if (pipelined && sweep_pipelined_fits(comp, n1, n2, s.nK)) {
       if constexpr (P::exact) launch_sweep64(s, comp, fwd, false, nslot, tab.p, st);
       else launch_sweep_pipelined(s, comp, fwd, nslot, st, sweep_vw, sweep_lines);
       return;
@@ -641,21 +665,15 @@ void Ops<P>::apply_aphi(const C* X, C* Y, int nslot, const int* sys_list, const 
   s.s33u = gu.s33;
   s.aphi_fix = aphi_fix ? 1 : 0;
   const int n1 = m->n1, n2 = m->n2, n3 = m->n3;
-  const bool lines = line_fits(n3);
-  const long sbs = sweep_split_scratch(n1, n2, n3);
+  const long sbs = sweep_line_scratch(n1, n2, n3);
+  const bool lines = line_fits(n3) && line_scratch(sbs, true);
   if constexpr (!P::exact) {
-    if (lines) {
-      sweep_scratch(sbs);
-      if (!rhs.p) rhs.alloc(sizeof(C) * (size_t)m->lE * nmax);
-      launch_line_bounds(s, nslot, st);
-    }
+    if (lines) launch_line_bounds(s, nslot, st);
   }
   if (!lines) zero(Y, m->lE, nslot, sys_list);
   launch_aphi_div<P>(s, BV.as<C>(), nslot, st);
   CSEM_CUDA_TRY(cudaMemsetAsync(V.p, 0, sizeof(C) * (size_t)m->lv * nslot, st));
-  if constexpr (P::exact) {
-    if (pipelined_sweeps) diag_table(s, nslot);
-  }
+  const bool pipelined = diag_table(s, nslot);
   // an edge sweep in one launch where the complex128 pipeline takes it, complex64 as LU-SGS's by
   // lines, else by diagonals
   auto edges = [&](int comp, bool fwd) {
@@ -669,7 +687,7 @@ void Ops<P>::apply_aphi(const C* X, C* Y, int nslot, const int* sys_list, const 
         return;
       }
     } else {
-      if (pipelined_sweeps && sweep_pipelined_fits(comp, n1, n2, n3)) {
+      if (pipelined && sweep_pipelined_fits(comp, n1, n2, n3)) {
         launch_sweep64(s, comp, fwd, true, nslot, tab.p, st);
         return;
       }

@@ -144,7 +144,7 @@ class Ops {
   // split sweeps with a warp per line in the row pipeline's place (k_lusgs6.cu), on one stream
   bool line_sweeps = true;
   bool line_fits(int nK) const;  // they are on and take this grid (nK: its planes)
-  bool line_fits() const { return line_fits(m->airbc ? m->n3f : m->n3); }
+  bool line_fits() const { return !no_room && line_fits(m->airbc ? m->n3f : m->n3); }  // LU-SGS's
   // whether the caller should number the groups within two halves of the slots
   bool halves() const { return split_sweeps && split_overlap && !line_fits(); }
   // split sweeps on two halves of the slots, one on `aux`, so that one half's passes can
@@ -186,10 +186,16 @@ class Ops {
   // sb for sbs entries a slot. LU-SGS with the air above the model sweeps more planes than A-phi,
   // so it may move
   void sweep_scratch(long sbs);
+  // sb for the line sweeps and, for A-phi, rhs. Where the device has no room for them left it is
+  // false from then on, and the sweeps that take less run (A-phi's by diagonals: nothing)
+  bool line_scratch(long sbs, bool aphi);
+  bool no_room = false, no_room_aphi = false;
   // counts what makes launches captured earlier other than those of now: sb moved, or one of the
   // options above changed
   unsigned epoch = 0;
-  void diag_table(const SweepP<P>& s, int nslot);  // complex128: the pipelined sweeps' diagonal table
+  // complex128: fills the pipelined sweeps' diagonal table; false without room for it (then, and
+  // with pipelined_sweeps off, the sweeps run by diagonals)
+  bool diag_table(const SweepP<P>& s, int nslot);
   int split_ctas() const;  // the split pipelines' grid cap on two streams: split_cap CTAs per SM (0: none)
   ~Ops();
 };

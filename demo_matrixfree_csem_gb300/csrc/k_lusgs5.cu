@@ -369,16 +369,12 @@ __global__ void CSEM_SWEEP_BOUNDS_S(VW, NW) k_sweep_eyz32s(SweepP<F32> s, const 
   }
 }
 
-// entries per slot that the pass stores: the largest component's on the sweep grid, or the
-// largest component's lines as streams (k_lusgs6.cu)
+// entries per slot that the pass stores: the largest component's on the sweep grid
 long sweep_split_scratch(int n1, int n2, int nK)
 {
   const long a = (long)n1 * (n2 + 1) * (nK + 1), b = (long)(n1 + 1) * n2 * (nK + 1),
              c = (long)(n1 + 1) * (n2 + 1) * nK;
-  const int sk = line_steps(nK - 1), sj = line_steps(n2 - 1);
-  const long d = (long)line_entry(line_strips(n2 - 1), sk, n1, 0, 0), e = (long)line_entry(line_strips(n1 - 1), sk, n2, 0, 0),
-             f = (long)line_entry(line_strips(n1 - 1), sj, nK, 0, 0);
-  return (std::max(std::max(std::max(a, b), std::max(c, d)), std::max(e, f)) + 31) / 32 * 32;
+  return std::max(a, std::max(b, c));
 }
 
 template <int VW, int NW>

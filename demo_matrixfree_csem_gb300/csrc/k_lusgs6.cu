@@ -42,6 +42,7 @@
 // DRAM rate, bound by its loads' latency; the chain runs at 50% (large batches: 7 or 8 lines on
 // an SM by its shared memory, and its load and store unit) or is bound by its steps' latency, 640
 // cycles for 8 rows (small ones).
+#include <algorithm>
 #include <type_traits>
 #include "csem_cuda.cuh"
 #include "engine.h"
@@ -720,6 +721,15 @@ bool sweep_line_fits(int n1, int n2, int nK)
 {
   const double most = 8.0 * 3.0 * (n1 + 1.0) * (n2 + 1.0) * (nK + 1.0);
   return most < 4294967296.0 && n1 >= 2 && n2 >= 2 && nK >= 2 && line_smem<8, 4>(nK - 1) <= SMEM_MOST && line_smem<1, 8>(n2 - 1) <= SMEM_MOST;
+}
+
+// entries per slot: the largest component's lines as streams
+long sweep_line_scratch(int n1, int n2, int nK)
+{
+  const int sk = line_steps(nK - 1), sj = line_steps(n2 - 1);
+  const size_t a = line_entry(line_strips(n2 - 1), sk, n1, 0, 0), b = line_entry(line_strips(n1 - 1), sk, n2, 0, 0),
+               c = line_entry(line_strips(n1 - 1), sj, nK, 0, 0);
+  return (long)std::max(a, std::max(b, c));
 }
 
 void launch_line_bounds(const SweepP<F32>& s, int nslot, cudaStream_t st)
