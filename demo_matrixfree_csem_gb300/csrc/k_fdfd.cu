@@ -128,20 +128,32 @@ k_fdfd(GridP<P> g, const SysScal<P>* __restrict__ scal, const typename P::C* __r
     return p;
   };
   PlaneIn nxt = load_plane(kb, oEx, oEy, oEz);
-  // imag: 1 / (i w mu0) is imaginary, as for real frequencies; it goes into the spacings'
-  // reciprocals, and H = i t: 54 FP64 operations a cell instead of 66, which bind this kernel (24
-  // systems of 3.7 M cells: 15.3 -> 14.3 ms with 8 rows a tile)
+  // imag: 1 / (i w mu0) is imaginary, as for real frequencies; divided by the spacings it takes their
+  // reciprocals' place, and H = i t: 53 FP64 operations a cell instead of 66, which bind this kernel
+  // (24 systems of 3.7 M cells: 15.3 -> 14.3 ms with 8 rows a tile). The quotients are rounded once,
+  // as they carry the same error into every point of a column or plane: those in z each lane forms
+  // for one of 32 planes
   auto march = [&](auto imag) {
     constexpr bool IMAG = decltype(imag)::value;
     auto times = [&](C t) { return IMAG ? P::mk(-t.y, t.x) : cmul<P>(t, iwmu); };
-    const R q1s = IMAG ? r1s * iwmu.y : r1s, q2s = IMAG ? r2s * iwmu.y : r2s;
+    auto quotient = [&](R d, R r) {
+      const R q = iwmu.y * r;
+      return fma(fma(-q, d, iwmu.y), r, q);
+    };
+    const R q1s = IMAG ? quotient(d1s, r1s) : r1s, q2s = IMAG ? quotient(d2s, r2s) : r2s;
+    R q3 = 0;
     for (int k = kb; k < ke; k++, oEx += sEx, oEy += sEy, oEz += sEz) {
       const int kf = k + ks;
       const int pb = k & 1;
       const bool kin = k < n3;
       const PlaneIn cur = nxt;
       if (k + 1 < ke) nxt = load_plane(k + 1, oEx + sEx, oEy + sEy, oEz + sEz);
-      const R d3s = g.d3s[kf], q3s = IMAG ? g.r3s[kf] * iwmu.y : g.r3s[kf], d3 = g.d3[kf], r3 = g.r3[kf];
+      const R d3s = g.d3s[kf], d3 = g.d3[kf], r3 = g.r3[kf];
+      if (IMAG && (k - kb & 31) == 0) {
+        const int kl = min(kf + lane, n3 + ks);
+        q3 = quotient(g.d3s[kl], g.r3s[kl]);
+      }
+      const R q3s = IMAG ? __shfl_sync(0xffffffffu, q3, k - kb & 31) : g.r3s[kf];
       const C ez = cur.ez, ezj = cur.ezj, exj = cur.exj, ex1 = cur.ex1, ey1 = cur.ey1;
       C ezi, eyi;  // Ez(k, j, i+1), Ey(k, j, i+1): the next lane's, loaded by the last lane
       ezi.x = __shfl_down_sync(0xffffffffu, ez.x, 1);
