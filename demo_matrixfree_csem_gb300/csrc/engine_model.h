@@ -127,10 +127,10 @@ class Ops {
   cudaStream_t st;
   DevBuf hz0, K, K2, ghx, ghy, cap, V, BV, scal, sb, tab, rhs;
   FftPlans* fft;
-  // LU-SGS sweeps: true = one pipelined-warp launch per component sweep (k_lusgs2.cu),
-  // false = one launch per wavefront diagonal (k_lusgs.cu); both give identical results
+  // Sweeps: true = one launch per component sweep (complex128: k_lusgs64.cu, complex64: by the
+  // options below), false = one launch per wavefront diagonal (k_lusgs.cu; complex128: the same bits)
   bool pipelined_sweeps = true;
-  int sweep_vw = 0;  // points per thread and step of the pipelined sweeps (0: default)
+  int sweep_vw = 0;  // complex64: points per thread and step of the pipelined sweeps (0: default)
   int sweep_lines = 1;  // complex64: lines one CTA of the pipelined sweeps carries as a conveyor
   // complex64: systems of one frequency one CTA of the pipelined sweeps carries (1, 2, 4);
   // used where the caller passes groups of 2 or 4 to apply_lusgs

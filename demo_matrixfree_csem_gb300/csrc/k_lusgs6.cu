@@ -37,7 +37,7 @@
 // entry per row and lane, 20 sectors a request, and join a line's warps by barriers at every
 // step. Per application, them, this with one warp to a line and one point to a pass's thread, and
 // this, one context: 200 x 140 x 140 cells, 48 systems 23.3, 14.6, 12.8 ms, 16 systems 8.02,
-// 5.30, 4.44, 3 systems 2.11, 1.40, 1.08; 84^3 cells, 6 systems 0.86, 0.51, 0.39; 81 x 73 x 67
+// 5.30, 4.42, 3 systems 2.11, 1.40, 1.07; 84^3 cells, 6 systems 0.86, 0.51, 0.39; 81 x 73 x 67
 // cells, 3 systems at 3 frequencies 0.51, 0.35, 0.25. The pass takes 60% of it, at 60% of the
 // DRAM rate, bound by its loads' latency; the chain runs at 50% (large batches: 7 or 8 lines on
 // an SM by its shared memory, and its load and store unit) or is bound by its steps' latency, 640
@@ -181,9 +181,9 @@ __device__ __forceinline__ C form_B(const Coef& c, C b, C kc)
 }
 
 constexpr int PASS_WARPS = 2;
-// Percent of an SM's 228 KB that the passes leave for shared memory (Ex's uses 34 KB). With the
-// chains' setting (all of it) the passes' loads miss L1: 16 systems 4.81 -> 6.38 ms an
-// application, and 6.04 where two contexts' applications overlap; so 4.81 and 4.60
+// Percent of an SM's 228 KB that the passes leave for shared memory (Ex's uses 26 KB). With the
+// chains' setting (all of it) the passes' loads miss L1: 16 systems 5.80 ms an application instead
+// of 4.42, and 5.53 instead of 4.25 where three contexts' applications overlap
 constexpr int PASS_SMEM = 20;
 
 }  // namespace

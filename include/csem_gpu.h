@@ -253,7 +253,9 @@ void *csem_ctx_stream(csem_ctx *c);
  *                     residuals r = b - A x with a complex128 stencil that multiplies by
  *                     reciprocal spacings and lets the compiler contract multiply-adds
  *                     (complex128 accuracy, not the reference's rounding: the defect
- *                     correction needs no more); 0: the bit-faithful complex128 stencil.
+ *                     correction needs no more), and with the airwave by line transforms
+ *                     on square uniform grids of 64, 256 or 1024 points a side; 0: the
+ *                     bit-faithful complex128 stencil and the airwave by cuFFT.
  *                     The complex128 solver (precision 64) and the operator entry points
  *                     always use the bit-faithful one;
  *   "fused_dots"      1: the batched complex64 BiCGStab forms v.r0 after v = A p and s.t,
@@ -298,7 +300,8 @@ void *csem_ctx_stream(csem_ctx *c);
  *                     depth (CTAs per SM 2, 4, 8); 0 (default): the fixed defaults.
  *                     complex64 results may then differ in the last bits from run to run,
  *                     so it is off by default;
- *   "stencil_by"      stencil tile height, output rows per CTA: 4, 8 (default) or 16;
+ *   "stencil_by"      stencil tile height, output rows per CTA: 4, 8 (default) or 16
+ *                     (the batched solve's complex128 residual: 16 where this is 8);
  *   "stencil_ctas"    CTAs per SM the stencil's plane chunks aim for (1..16, default 4),
  *                     which sets the z-block depth. Neither stencil option changes results;
  *   "graphs"          1 (default): the batched BiCGStab replays the iterations between
