@@ -19,6 +19,7 @@
 // loads and 64-bit addresses); tiles 4 and 16 rows high 850 and 1070 us. Of about 230
 // instructions a warp and plane 70 are arithmetic; registers (72, for three CTAs of 8 rows
 // on an SM) limit the loads in flight.
+#include <algorithm>
 #include <type_traits>
 #include "csem_cuda.cuh"
 #include "engine.h"
@@ -79,7 +80,7 @@ __global__ void __launch_bounds__(32 * (BY + 1), BY >= 16 ? 1 : (BY >= 8 ? 3 : 5
 {
   __shared__ float4 sH[2][BY + 1][32];  // (Hx, Hz) of each row
   const int lane = threadIdx.x, w = threadIdx.y;
-  const int i = blockIdx.x * 30 + lane - 1, j = blockIdx.y * BY + w - 1;
+  const int i = blockIdx.x * 30 + lane, j = blockIdx.y * BY + w - 1;
   const int slot = blockIdx.z / nkc, kc = blockIdx.z - slot * nkc;
   const int sys = sys_list ? sys_list[slot] : slot;
   const int n1 = g.n1, n2 = g.n2, n3 = g.n3, ks = g.kstart;
@@ -97,8 +98,10 @@ __global__ void __launch_bounds__(32 * (BY + 1), BY >= 16 ? 1 : (BY >= 8 ? 3 : 5
   const char* const s22 = (const char*)(g.s22) + (size_t)ks * (sY / 2);
   const char* const s33 = (const char*)(g.s33) + (size_t)ks * (sZ / 2);
   // the nearest column that each component has
-  const int ix = min(max(i, 0), n1 - 1), iy = min(max(i, 0), n1), jx = min(max(j, 0), n2), jy = min(jx, n2 - 1);
-  const bool mine = lane >= 1 && lane <= 30 && w >= 1 && i <= n1 && j <= n2;
+  const int ix = min(i, n1 - 1), iy = min(i, n1), jx = min(max(j, 0), n2), jy = min(jx, n2 - 1);
+  // column 0 has no left neighbour that counts and column n1 holds zeros only: both come with the
+  // first and the last tile, on the lanes that are else extra
+  const bool mine = (lane >= 1 || i == 0) && (lane <= 30 || i == n1) && w >= 1 && i <= n1 && j <= n2;
   const bool outX = mine && i < n1, outY = mine && j < n2, outZ = mine;
   const bool inX = j >= 1 && j <= n2 - 1, inY = i >= 1 && i <= n1 - 1, inZ = inX && inY;
   Off oX = point_offset<Off>(ix, jx, kb, n1, sX), oY = point_offset<Off>(iy, jy, kb, n1 + 1, sY),
@@ -220,12 +223,19 @@ __global__ void __launch_bounds__(32 * (BY + 1), BY >= 16 ? 1 : (BY >= 8 ? 3 : 5
 
 namespace {
 
+// tiles for columns 1 .. n1 - 1 (a tile more for column 0 or n1 alone made n1 = 30 and 61 slower than
+// tiles of 31 did: 30 x 140 x 120 cells, 6 systems, 88 us with those, 105 with the second tile, 67 now)
+FdfdShape shape(int n1, int n2, int n3, int nsys, int by, int ctas_per_sm)
+{
+  return fdfd_shape(std::max(n1 - 2, 0), n2, n3, nsys, by, ctas_per_sm, FDFD32_TILE);
+}
+
 template <int EPI>
 void launch_by(const GridP<F32>& g, const SysScal<F32>* scal, const C* X, C* Y, const C* ghx, const C* ghy, int nsys,
                const int* sys_list, cudaStream_t st, int by, int ctas_per_sm, const C* E, double2* part)
 {
   if (by != 4 && by != 16) by = 8;
-  const FdfdShape f = fdfd_shape(g.n1, g.n2, g.n3, nsys, by, ctas_per_sm, FDFD32_TILE);
+  const FdfdShape f = shape(g.n1, g.n2, g.n3, nsys, by, ctas_per_sm);
   dim3 blk(32, by + 1), grd(f.gx, f.gy, nsys * f.nkc);
   auto go = [&](auto tile, auto off) {
     constexpr int BY = decltype(tile)::value;
@@ -262,7 +272,7 @@ void launch_fdfd_dot(const GridP<F32>& g, const SysScal<F32>* scal, const float2
 
 int fdfd_partials(int n1, int n2, int n3, int nsys, int by, int ctas_per_sm)
 {
-  const FdfdShape f = fdfd_shape(n1, n2, n3, nsys, by, ctas_per_sm, FDFD32_TILE);
+  const FdfdShape f = shape(n1, n2, n3, nsys, by, ctas_per_sm);
   return f.gx * f.gy * f.nkc;
 }
 
