@@ -8,6 +8,7 @@
 // summed per thread with a compensated (TwoSum) float pair, so the per-thread partials
 // carry ~48 significant bits; partials are combined in FP64.
 #include <cooperative_groups.h>
+#include <algorithm>
 #include <type_traits>
 #include "csem_cuda.cuh"
 #include "engine.h"
@@ -355,13 +356,25 @@ void launch_res_norm(long n, int nslot, const int* sys_list, const double2* b, c
   count_launch(), k_dot_final<<<nslot, DOT_THREADS, 0, st>>>(partial, nblk, out);
 }
 
+// How many vectors of nblk blocks take the one launch of a cluster each: beyond, its 8 blocks a vector
+// take more rounds of the SMs than k_dot_partial's nblk (1000 values: 128 vectors 8.3 us against 10.4,
+// 152 vectors 11.9 against 10.4, 2000 vectors 66 against 38; 12000: 64 vectors 12.4 against 12.6, 76
+// 14.4 against 13.6). complex128 products are bound by the FP64 unit, and at one block to an SM 14
+// clusters fit the chip (16384 values: 14 vectors 12.4 us against 14.4, 16 16.5 against 14.4; 14000:
+// 32 vectors 16.5 against 20.6, 40 22.7 against 20.6)
+template <class Acc> static int short_dots(int nblk)
+{
+  if (std::is_same<Acc, DotAcc<F64>>::value && nblk >= 7) return nblk == 7 ? 32 : 14;
+  return std::min(128, 384 / nblk);
+}
+
 template <class P, class Acc>
 static void launch_dot_of(const typename P::C* a, const typename P::C* b, long n, long stride, int nslot,
                           const int* sys_list, double2* partial, int nblk, double2* out, cudaStream_t st)
 {
   const dim3 grd(nblk, nslot);
   count_launch();
-  if (nblk <= DOT_CLUSTER) {
+  if (nblk <= DOT_CLUSTER && nslot <= short_dots<Acc>(nblk)) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(DOT_CLUSTER, nslot);
     cfg.blockDim = dim3(32 * nblk);
